@@ -168,7 +168,9 @@ void plan_setup( SetupArgs const &a, int precision, uint8_t const *basis_of_grou
     plan.bucket_start.allocate( N_KEYS, s );
     plan.bucket_task.allocate( N_KEYS, s );
     plan.tasks.allocate( ( n + 31 ) / 32 + N_KEYS, s );
-    plan.counter.allocate( 1, s );
+    plan.rest_task.allocate( ( n + 31 ) / 32 + N_KEYS, s );
+    plan.rest_list.allocate( std::max<int64_t>( 1, n ), s );
+    plan.counters.allocate( 1, s );
     DTK_CUDA_OR_THROW( cudaMemsetAsync( plan.hist.get(), 0, N_KEYS * sizeof( unsigned ), s ) );
     if ( n )
     {
@@ -214,7 +216,9 @@ BatchSetupArgs batch_args( SetupArgs const &a, SetupPlan &plan, double *u_work )
     b.underdetermined = a.underdetermined;
     b.rotations = a.rotations;
     b.status = a.status;
-    b.counter = plan.counter.get();
+    b.counters = plan.counters.get();
+    b.rest_list = plan.rest_list.get();
+    b.rest_task = plan.rest_task.get();
     b.u_work = u_work;
     return b;
 }
@@ -236,7 +240,7 @@ void tune_setup( SetupArgs const &a, SetupPlan &plan, double *u_work, cudaStream
     int64_t pf[N_PATH + 1];
     DTK_CUDA_OR_THROW( cudaMemcpyAsync( pf, plan.path_first.get(), sizeof( pf ), cudaMemcpyDeviceToHost, s ) );
     DTK_CUDA_OR_THROW( cudaStreamSynchronize( s ) );
-    int64_t const wave = batch_setup_threads() / 32; // resident warps
+    int64_t const wave = (int64_t)batch_fixed_warps(); // resident warps
     cudaEvent_t e0, e1;
     DTK_CUDA_OR_THROW( cudaEventCreate( &e0 ) );
     DTK_CUDA_OR_THROW( cudaEventCreate( &e1 ) );
@@ -320,7 +324,7 @@ void run_setup_plan( SetupArgs const &a, int precision, uint8_t const *basis_of_
     if ( a.n_tgt == 0 )
         return;
     if ( !plan.u_work.get() )
-        plan.u_work.allocate( (size_t)jacobi_work_doubles( BS_MAX_M ) * batch_setup_threads(), s );
+        plan.u_work.allocate( batch_work_doubles(), s );
     // the tasks exist before any launch reads them (the tuner's samples
     // too); refilled with the tuned lane counts.  The statistics counters
     // collect the sample runs as well: zeroed after them
@@ -531,8 +535,8 @@ struct dtk_mls_batch_s
     ~dtk_mls_batch_s()
     {
         life.retire( offset, idx, coeff64, coeff32, rows, tasks, status, counters, plan.list, plan.hist,
-                     plan.n_tasks, plan.path_first, plan.bucket_start, plan.bucket_task, plan.tasks, plan.counter,
-                     plan.u_work );
+                     plan.n_tasks, plan.path_first, plan.bucket_start, plan.bucket_task, plan.tasks, plan.rest_task,
+                     plan.rest_list, plan.counters, plan.u_work );
         if ( exec )
             cudaGraphExecDestroy( exec );
         if ( graph )

@@ -556,13 +556,23 @@ struct SetupArgs
     unsigned *status;
 };
 void setup_fp64( SetupArgs const &a, cudaStream_t s );
+// The FP64 form with the Jacobi in fixed point (weights >= 0 only:
+// fixed_supported); the targets it hands back go to list[0 .. *count), zeroed
+// by the caller.  `work` holds fixed_work_doubles doubles.
+__host__ __device__ constexpr bool fixed_supported( int rbf )
+{
+    return rbf < DTK_BUHMANN2; // positive weights: a positive semi-definite moment matrix
+}
+size_t fixed_work_doubles( int64_t n_tgt );
+void setup_fixed( SetupArgs const &a, double *work, uint32_t *list, unsigned *count, cudaStream_t s );
 void setup_mixed( SetupArgs const &a, cudaStream_t s );
 constexpr int FUSED_MAX_ROW = 32; // longest row the fused one-thread-per-target kernels take
 
-// Persistent batched setup (FP64 Jacobi): the targets of a bucketed list in
-// tasks of up to 32 targets of one bucket, taken by warps from a counter.
+// Persistent batched setup (FP64 form): the targets of a bucketed list in
+// tasks of up to 32 targets of one bucket, taken by warps from a counter; one
+// launch with the Jacobi in fixed point, one in FP64 over what that hands back.
 constexpr int SETUP_RBFS = 9, SETUP_PATHS = 3, SETUP_KEYS = 3 * SETUP_RBFS * SETUP_PATHS;
-constexpr int BS_WARPS = 8; // warps a block of the persistent setup (one block an SM)
+constexpr int BS_WARPS = 8; // warps a block of the FP64 launch (one block an SM)
 struct SetupTask
 {
     int32_t first; // the task's first target in the bucketed list
@@ -598,13 +608,30 @@ struct BatchSetupArgs
     float *coeff32 = nullptr;
     unsigned long long *underdetermined, *rotations;
     unsigned *status;
-    unsigned *counter; // zeroed by batch_setup before the launch
-    double *u_work;    // jacobi_work_doubles( BS_MAX_M ) doubles per thread of the grid (batch_setup_threads)
+    // zeroed by batch_setup before the launches: the task counters of the
+    // fixed-point and the FP64 launch, and what the first hands to the second
+    struct Counters
+    {
+        int64_t rest_tasks;
+        unsigned task[2];
+        unsigned rest; // targets
+        unsigned pad;
+    } * counters;
+    // the targets handed back (n_list entries) and their tasks (as many as
+    // `tasks`)
+    uint32_t *rest_list;
+    SetupTask *rest_task;
+    double *u_work; // batch_work_doubles()
     unsigned jcap[3] = {0, 0, 0};
     int jlog = JACOBI_LOG;
 };
 void batch_setup( BatchSetupArgs const &a, cudaStream_t s );
-int64_t batch_setup_threads();
+// Its fixed-point launch (dtk_setup_fixed.cu), the warps of its grid and its
+// work area.
+void batch_fixed( BatchSetupArgs const &a, cudaStream_t s );
+size_t batch_fixed_warps();
+size_t batch_fixed_work_doubles();
+size_t batch_work_doubles(); // the work area of both launches
 
 // The device plan of a setup over targets of mixed classes (kept by a batch
 // handle for its re-setups): the targets in bucket order, the bucket sizes,
@@ -619,8 +646,9 @@ struct SetupPlan
     DeviceBuffer<uint32_t> list;       // targets, bucket order
     DeviceBuffer<unsigned> hist;       // targets per bucket
     DeviceBuffer<int64_t> n_tasks, path_first, bucket_start, bucket_task;
-    DeviceBuffer<SetupTask> tasks;
-    DeviceBuffer<unsigned> counter;
+    DeviceBuffer<SetupTask> tasks, rest_task;
+    DeviceBuffer<uint32_t> rest_list;
+    DeviceBuffer<BatchSetupArgs::Counters> counters;
     DeviceBuffer<double> u_work;
     struct Bucket
     {

@@ -1,4 +1,6 @@
-// Fused MLS setup, FP64 form (sm_103a).
+// Fused MLS setup, FP64 form (sm_103a): the kernels that run the reference's
+// Jacobi in FP64, for the Buhmann functions (their weights change sign) and for
+// the targets that the fixed-point kernels (dtk_setup_fixed.cu) hand back.
 //
 // One thread per target (targets in Morton order) runs every stage of the
 // reference constructor after the search, fused, with nothing but the
@@ -532,9 +534,12 @@ __global__ void __launch_bounds__( FP64_THREADS, 1 )
     k_setup_fp64( Neighbours nb, PointsView tgt, int32_t const *offset,
                   uint32_t const *order, int64_t n_tgt, int rbf, bool rows_sorted,
                   double *coeff, unsigned long long *under_count,
-                  unsigned long long *rot_count, unsigned *status, unsigned jcap, int jlog, double *u_work )
+                  unsigned long long *rot_count, unsigned *status, unsigned jcap, int jlog, double *u_work,
+                  unsigned const *n_listed )
 {
     extern __shared__ double smem[];
+    if ( n_listed ) // the targets order[0 .. *n_listed)
+        n_tgt = *n_listed;
     int const nt = blockDim.x; // FP64_THREADS, or 32 when the targets are few
     int64_t const T = (int64_t)gridDim.x * nt;
     int64_t const tid = blockIdx.x * (int64_t)nt + threadIdx.x;
@@ -754,8 +759,9 @@ __global__ void k_svd_general( int n, int64_t count, double const *a, double *pi
 }
 
 // ---------------------------------------------------------------------------
-// Persistent batched setup: every FP64-Jacobi target of a batch, of any
-// (basis, rbf) and row length, in one launch.  A warp takes tasks from a
+// Persistent batched setup, FP64 Jacobi: the targets of a batch that the
+// fixed-point launch (dtk_setup_fixed.cu) hands back, of any (basis, rbf) and
+// row length, in one launch.  A warp takes tasks from a
 // counter; a task is up to 32 targets of one bucket (same basis and rbf) and
 // a lane count G: G lanes per target gather the neighbours for the radius and
 // the moments (sums combined by shuffles in the group), the moments go to the
@@ -930,7 +936,7 @@ __global__ void __launch_bounds__( BS_WARPS * 32, 1 ) k_batch_setup( BatchSetupA
     {
         unsigned c = 0;
         if ( lane == 0 )
-            c = atomicAdd( a.counter, 1u );
+            c = atomicAdd( &a.counters->task[1], 1u );
         int64_t const ti = a.t_begin + __shfl_sync( FULL, c, 0 );
         if ( ti >= t_end )
             break;
@@ -968,19 +974,41 @@ __global__ void __launch_bounds__( BS_WARPS * 32, 1 ) k_batch_setup( BatchSetupA
     }
 }
 
+// n_listed (device, null: all): the targets a.order[0 .. *n_listed) only,
+// one warp a block so that a few of them spread over the SMs.
 template <int M>
-void launch_fp64( SetupArgs const &a, cudaStream_t s )
+void launch_fp64( SetupArgs const &a, DeviceBuffer<double> &work, unsigned const *n_listed, cudaStream_t s )
 {
-    JacobiGrid const jg = jacobi_grid<M>( a.n_tgt );
+    JacobiGrid jg = jacobi_grid<M>( n_listed ? std::min<int64_t>( a.n_tgt, 1 ) : a.n_tgt );
+    if ( n_listed )
+        jg.blocks = (unsigned)std::min<int64_t>( ( a.n_tgt + 31 ) / 32, FP64_THREADS / 32 * (int64_t)num_sms() );
     ensure_dynamic_smem( k_setup_fp64<M>, jg.smem );
-    DeviceBuffer<double> u_work( (size_t)jacobi_work_doubles( M ) * jg.threads * jg.blocks, s );
+    size_t const need = (size_t)jacobi_work_doubles( M ) * jg.threads * jg.blocks;
+    if ( !n_listed )
+        work.allocate( need, s );
     Neighbours const nb{a.src, a.idx, a.pos, a.s2};
     k_setup_fp64<M><<<jg.blocks, jg.threads, jg.smem, s>>>( nb, a.tgt, a.offset, a.order,
                                                          a.n_tgt, a.rbf, a.rows_sorted, a.coeff64,
                                                          a.underdetermined, a.rotations, a.status,
                                                          (unsigned)jacobi_cap( M ), jacobi_log_cap(),
-                                                         u_work.get() );
+                                                         work.get(), n_listed );
     check_launch( "k_setup_fp64" );
+}
+
+void setup_fp64_over( SetupArgs const &a, DeviceBuffer<double> &work, unsigned const *n_listed, cudaStream_t s )
+{
+    switch ( a.basis )
+    {
+    case DTK_CONSTANT3:
+        launch_fp64<1>( a, work, n_listed, s );
+        break;
+    case DTK_LINEAR3:
+        launch_fp64<4>( a, work, n_listed, s );
+        break;
+    default:
+        launch_fp64<10>( a, work, n_listed, s );
+        break;
+    }
 }
 
 } // namespace
@@ -990,18 +1018,26 @@ void setup_fp64( SetupArgs const &a, cudaStream_t s )
     NvtxRange const nvtx_range( "DTK_compute_polynomial_coeffs" );
     if ( a.n_tgt == 0 )
         return;
-    switch ( a.basis )
+    DeviceBuffer<double> work;
+    if ( !fixed_supported( a.rbf ) )
     {
-    case DTK_CONSTANT3:
-        launch_fp64<1>( a, s );
-        break;
-    case DTK_LINEAR3:
-        launch_fp64<4>( a, s );
-        break;
-    default:
-        launch_fp64<10>( a, s );
-        break;
+        setup_fp64_over( a, work, nullptr, s );
+        return;
     }
+    // the fixed-point kernel, then the FP64 one over the targets it handed
+    // back (their number stays on the device); one work area for both
+    DeviceBuffer<uint32_t> list( a.n_tgt, s );
+    DeviceBuffer<unsigned> count( 1, s );
+    DTK_CUDA_OR_THROW( cudaMemsetAsync( count.get(), 0, sizeof( unsigned ), s ) );
+    int64_t const warps = ( a.n_tgt + 31 ) / 32;
+    work.allocate( std::max<size_t>( fixed_work_doubles( a.n_tgt ),
+                                     jacobi_work_doubles( basis_size( a.basis ) ) *
+                                         (size_t)std::min<int64_t>( warps * 32, FP64_THREADS * (int64_t)num_sms() ) ),
+                   s );
+    setup_fixed( a, work.get(), list.get(), count.get(), s );
+    SetupArgs rest = a;
+    rest.order = list.get();
+    setup_fp64_over( rest, work, count.get(), s );
 }
 
 size_t batch_setup_smem()
@@ -1009,9 +1045,10 @@ size_t batch_setup_smem()
     return (size_t)BS_WARPS * BS_SLOT * sizeof( double );
 }
 
-int64_t batch_setup_threads()
+size_t batch_work_doubles()
 {
-    return (int64_t)num_sms() * BS_WARPS * 32;
+    return std::max<size_t>( batch_fixed_work_doubles(),
+                             (size_t)jacobi_work_doubles( BS_MAX_M ) * num_sms() * BS_WARPS * 32 );
 }
 
 void batch_setup( BatchSetupArgs const &args, cudaStream_t s )
@@ -1022,8 +1059,16 @@ void batch_setup( BatchSetupArgs const &args, cudaStream_t s )
     a.jcap[1] = (unsigned)jacobi_cap( 4 );
     a.jcap[2] = (unsigned)jacobi_cap( 10 );
     a.jlog = jacobi_log_cap();
+    DTK_CUDA_OR_THROW( cudaMemsetAsync( a.counters, 0, sizeof( *a.counters ), s ) );
+    batch_fixed( a, s );
+    // the FP64 launch over the targets left, each with its task's lanes
+    a.list = a.rest_list;
+    a.tasks = a.rest_task;
+    a.n_tasks = &a.counters->rest_tasks;
+    a.t_begin = 0;
+    a.t_end = -1;
+    a.force_lanes = 0;
     ensure_dynamic_smem( k_batch_setup, batch_setup_smem() );
-    DTK_CUDA_OR_THROW( cudaMemsetAsync( a.counter, 0, sizeof( unsigned ), s ) );
     k_batch_setup<<<(unsigned)num_sms(), BS_WARPS * 32, batch_setup_smem(), s>>>( a );
     check_launch( "k_batch_setup" );
 }
