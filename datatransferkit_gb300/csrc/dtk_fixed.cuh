@@ -39,7 +39,7 @@ namespace dtk
 {
 
 constexpr int FX_DIGIT = 29;
-constexpr int FX_MASK = ( 1 << FX_DIGIT ) - 1;
+constexpr int FX_MASK = ( 1 << FX_DIGIT ) - 1, FX_HALF = 1 << ( FX_DIGIT - 1 );
 constexpr int FX_ONE = 60;  // the two leading digits as an integer: 2^60 is 1
 constexpr int FX_COEF = 58; // rotation factors: 2^58 is 1
 constexpr int FX_V = 54;    // column 0 of V (two digits): 2^54 is 1 at row 0's scale (headroom 64)
@@ -152,20 +152,31 @@ __host__ __device__ __forceinline__ uint64_t fx_inv_sqrt( uint64_t rho )
     return (uint64_t)( ( (int64_t)g << 32 ) + gc );
 }
 
-// A number of D = 2 or 3 digits: d[0] signed, the others in [0, 2^29).
+// A number of D = 2 or 3 digits: d[0] signed, the others balanced, in [-2^28,
+// 2^28), so that a small value of either sign has small digits (its magnitude
+// as a float needs no sign handling).
 template <int D>
 struct FxNum
 {
     int32_t d[D];
 };
-// A rotation factor: hi signed, lo in [0, 2^29).
+// the balanced low digit of v, and v without it
+__host__ __device__ __forceinline__ int32_t fx_low( int64_t v )
+{
+    return (int32_t)( (uint32_t)v << ( 32 - FX_DIGIT ) ) >> ( 32 - FX_DIGIT );
+}
+__host__ __device__ __forceinline__ int32_t fx_high( int64_t v )
+{
+    return (int32_t)( ( v + FX_HALF ) >> FX_DIGIT );
+}
+// A rotation factor.
 struct FxCoef
 {
     int32_t hi, lo;
 };
 __host__ __device__ __forceinline__ FxCoef fx_coef( int64_t v )
 {
-    return FxCoef{(int32_t)( v >> FX_DIGIT ), (int32_t)v & FX_MASK};
+    return FxCoef{fx_high( v ), fx_low( v )};
 }
 // the leading 60 bits as an integer (2^60 is 1)
 template <int D>
@@ -182,81 +193,89 @@ template <int D>
 __host__ __device__ __forceinline__ FxNum<D> fx_num( int64_t lead, int32_t last = 0 )
 {
     FxNum<D> x;
-    x.d[0] = (int32_t)( lead >> FX_DIGIT );
-    x.d[1] = (int32_t)lead & FX_MASK;
+    x.d[0] = fx_high( lead );
+    x.d[1] = fx_low( lead );
     if constexpr ( D == 3 )
         x.d[2] = last;
     return x;
 }
-// a x + b y: six (D = 2) or ten IMAD.WIDE.  The offset 2^29 in the lowest
-// column centres the error (the product of the lowest digits, on average a
-// quarter unit each, and the floor).  fits: the result is within the leading
-// digit.
+// a x + b y, rounded (without the product of the lowest digits, below half a
+// unit each): six (D = 2) or ten IMAD.WIDE.  Each column carries FX_HALF into
+// the next, so that a digit is its low 29 bits less FX_HALF; the constant 2^57
+// in a column is that carry.  fits: the result is within the leading digit.
 template <int D>
 __host__ __device__ __forceinline__ FxNum<D> fx_dot( FxCoef a, FxNum<D> const &x, FxCoef b, FxNum<D> const &y,
                                                      bool &fits )
 {
-    int64_t carry = 1 << FX_DIGIT;
+    constexpr int64_t HALF = FX_HALF, CARRY = (int64_t)FX_HALF << FX_DIGIT;
+    int64_t low = HALF + CARRY;
     if constexpr ( D == 3 )
-        carry = fx_mad( b.lo, y.d[1],
-                        fx_mad( b.hi, y.d[2], fx_mad( a.lo, x.d[1], fx_mad( a.hi, x.d[2], carry ) ) ) ) >>
-                FX_DIGIT;
+        low = ( fx_mad( b.lo, y.d[1],
+                        fx_mad( b.hi, y.d[2], fx_mad( a.lo, x.d[1], fx_mad( a.hi, x.d[2], low ) ) ) ) >>
+                FX_DIGIT ) +
+              CARRY;
     int64_t const m =
-        fx_mad( b.lo, y.d[0], fx_mad( b.hi, y.d[1], fx_mad( a.lo, x.d[0], fx_mad( a.hi, x.d[1], carry ) ) ) );
+        fx_mad( b.lo, y.d[0], fx_mad( b.hi, y.d[1], fx_mad( a.lo, x.d[0], fx_mad( a.hi, x.d[1], low ) ) ) );
     int64_t const h = fx_mad( b.hi, y.d[0], fx_mad( a.hi, x.d[0], m >> FX_DIGIT ) );
     fits = ( h >> FX_ONE ) == ( h >> 63 );
-    return fx_num<D>( h, (int32_t)m & FX_MASK );
+    FxNum<D> r;
+    r.d[0] = (int32_t)( h >> FX_DIGIT );
+    r.d[1] = ( (int32_t)h & FX_MASK ) - FX_HALF;
+    if constexpr ( D == 3 )
+        r.d[2] = ( (int32_t)m & FX_MASK ) - FX_HALF;
+    return r;
 }
-// |x| (or a unit less, for negative x) as a float in units of its last digit
+// x as a float in units of its last digit (relative error below 2^-22)
 template <int D>
-__host__ __device__ __forceinline__ float fx_abs_float( FxNum<D> const &x )
+__host__ __device__ __forceinline__ float fx_float( FxNum<D> const &x )
 {
-    int32_t const sign = x.d[0] >> 31, low = sign & FX_MASK;
-    float f = (float)( x.d[0] ^ sign );
+    float f = (float)x.d[0];
 #pragma unroll
     for ( int k = 1; k < D; ++k )
-        f = fx_fma( f, 536870912.f, (float)( x.d[k] ^ low ) );
+        f = fx_fma( f, 536870912.f, (float)x.d[k] ); // 2^29
     return f;
+}
+template <int D>
+__host__ __device__ __forceinline__ bool fx_zero( FxNum<D> const &x )
+{
+    return ( x.d[0] | x.d[1] | fx_last( x ) ) == 0;
+}
+// x's magnitude is at most FX_NOISE units of its last digit
+__host__ __device__ __forceinline__ bool fx_noise( FxNum<3> const &x )
+{
+    return ( x.d[0] | x.d[1] ) == 0 && (uint32_t)( x.d[2] + FX_NOISE ) <= 2u * FX_NOISE;
 }
 // |x| = m 2^(-e - 60) with 2^62 <= m < 2^63 (x not zero; m truncated)
 template <int D>
-__host__ __device__ __forceinline__ uint64_t fx_normal( FxNum<D> const &x, int &e )
+__host__ __device__ __forceinline__ uint64_t fx_normal( FxNum<D> const &x, int &e, bool &negative )
 {
     int64_t lead = fx_lead( x );
     int32_t last = fx_last( x );
-    if ( lead < 0 )
+    negative = lead < 0 || ( lead == 0 && last < 0 );
+    if ( negative )
     {
+        lead = -lead;
         last = -last;
-        lead = -lead - ( last < 0 ); // a digit of 2^29 is borrowed
-        last &= FX_MASK;
     }
-    if ( D == 3 && lead == 0 )
+    if ( D == 3 && lead <= 1 )
     {
-        int const z = fx_clz( (uint64_t)last ) - 1;
+        // the last digit leads, or decides whether the 1 above it stays
+        uint64_t const v = ( (uint64_t)lead << FX_DIGIT ) + (int64_t)last;
+        int const z = fx_clz( v ) - 1;
         e = z + FX_DIGIT;
-        return (uint64_t)last << ( z & 63 );
+        return v << ( z & 63 );
     }
+    // (a negative last digit below a power of two takes one from its bits)
+    lead -= D == 3 && last < 0;
     int const z = fx_clz( (uint64_t)lead ) - 1;
     e = z;
     uint64_t const m = (uint64_t)lead << ( z & 63 );
     if constexpr ( D == 2 )
         return m;
+    last &= FX_MASK;
     // as many of the last digit's bits as fit below the lead's
     return m + ( z >= FX_DIGIT ? (uint64_t)last << ( ( z - FX_DIGIT ) & 63 )
                                : (uint64_t)( last >> ( ( FX_DIGIT - z ) & 31 ) ) );
-}
-// x's magnitude is at most FX_NOISE units of its last digit
-template <int D>
-__host__ __device__ __forceinline__ bool fx_noise( FxNum<D> const &x )
-{
-    if ( D == 3 && x.d[1] != ( x.d[0] & FX_MASK ) )
-        return false; // the leading digits are not a sign
-    return x.d[0] == 0 ? x.d[D - 1] <= FX_NOISE : x.d[0] == -1 && x.d[D - 1] >= FX_MASK + 1 - FX_NOISE;
-}
-template <int D>
-__host__ __device__ __forceinline__ bool fx_zero( FxNum<D> const &x )
-{
-    return fx_lead( x ) == 0 && fx_last( x ) == 0;
 }
 
 // The rotation of one pivot block: the row with the larger diagonal entry is
@@ -368,6 +387,15 @@ struct FxLayout
         bool const flip = d > HALF || ( d == HALF && i >= HALF );
         return ( ( flip ? M - d : d ) - 1 ) * M + ( flip ? j : i );
     }
+    // the slots of {p, j} and {q, j}, j the t-th index past p and q
+    __host__ __device__ __forceinline__ static void column( int p, int q, int t, int &up, int &uq )
+    {
+        int j = t;
+        j += j >= p;
+        j += j >= q;
+        up = pair( p, j );
+        uq = pair( q, j );
+    }
     // the pair of a slot, p < q
     __host__ __device__ __forceinline__ static void of_slot( int u, int &p, int &q )
     {
@@ -383,14 +411,15 @@ struct FxLayout
 // fx_load); then f(u) / set_f(u, x) the off-diagonal numbers, diag(k) /
 // set_diag(k, x) the diagonal's leads, v(k) / set_v(k, x) column 0 of V and, at
 // the end and in its place, w(k) = V(k) / E(k, k); exp(k) / set_exp(k, d) the
-// rows' exponents; log(r, c, s, ls) rotation r: ls = 16 L + S, the rows before
+// rows' exponents; column(u, p, q, t, up, uq) is FxLayout's, u being the slot of
+// {p, q}; log(r, c, s, ls) rotation r: ls = 16 L + S, the rows before
 // it (the new rows are min(L, S) = X, max(L, S) = Y).  for_parts(fn) runs fn(h)
 // for the parts of this lane; merge(k1, k2, sum) combines a scan with the
 // other lane's; both(x) is x of all the matrix's lanes; sync() orders their
 // accesses.
 
-// the scale of row exponent d as a float: fx_abs_float( F(i, j) ) fx_scale( d_i )
-// fx_scale( d_j ) is |E(i, j)| times 2^29
+// the scale of row exponent d as a float: fx_float( F(i, j) ) fx_scale( d_i )
+// fx_scale( d_j ) is E(i, j) times 2^29
 __host__ __device__ __forceinline__ float fx_scale( int d )
 {
     return fx_pow2( d - 30 );
@@ -444,11 +473,15 @@ __host__ __device__ __forceinline__ bool fx_load( State const &st, bool live )
                 st.set_diag( p, lead );
                 continue;
             }
+            if ( low >= FX_HALF )
+            {
+                low -= 1 << FX_DIGIT;
+                ++lead;
+            }
             if ( bits & SIGN_BIT )
             {
                 low = -low;
-                lead = -lead - ( low < 0 );
-                low &= FX_MASK;
+                lead = -lead;
             }
             st.set_f( u, fx_num<3>( lead, low ) );
         }
@@ -473,7 +506,8 @@ __host__ __device__ __noinline__ int fx_exact_pivot( State const st )
             if ( fx_zero( f ) )
                 continue;
             int z;
-            uint64_t const m = fx_normal( f, z );
+            bool negative;
+            uint64_t const m = fx_normal( f, z, negative );
             int const e = st.exp( i ) + st.exp( j ) - z;
             if ( e > be || ( e == be && m > bm ) )
             {
@@ -497,8 +531,9 @@ __host__ __device__ __noinline__ bool fx_exact_go( State const st )
         if ( fx_zero( f ) )
             continue;
         int z, p, q;
+        bool negative;
         FxLayout<M>::of_slot( u, p, q );
-        uint64_t const m = fx_normal( f, z );
+        uint64_t const m = fx_normal( f, z, negative );
         double const e = fx_double( m, st.exp( p ) + st.exp( q ) - z - FX_ONE, false );
         acc += e * e;
     }
@@ -524,9 +559,9 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
         if ( live )
             st.for_parts( [&]( int h ) {
                 auto visit = [&]( int u, float si, float sj, bool mine ) {
-                    float const m = mine ? fx_abs_float( st.f( u ) ) * si * sj : 0.f;
+                    float const m = mine ? fx_float( st.f( u ) ) * si * sj : 0.f;
                     sum = fx_fma( m, m, sum );
-                    int const key = ( fx_float_bits( m ) & ~63 ) | u;
+                    int const key = ( fx_float_bits( m ) & 0x7fffffc0 ) | u;
                     int const lo = k1 < key ? k1 : key;
                     k2 = k2 > lo ? k2 : lo;
                     k1 = k1 > key ? k1 : key;
@@ -566,7 +601,6 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
             u = fx_exact_pivot<M>( st );
         int p, q;
         Lay::of_slot( u, p, q );
-        u = Lay::pair( p, q );
         FxNum<3> const fpq = st.f( u );
         // (the largest entry is this form's rounding: made zero below)
         bool const noise = go && fx_noise( fpq );
@@ -587,24 +621,20 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
             bool const swap = k >= 0 ? (uint64_t)fpp < fx_shr( (uint64_t)fqq, 2 * k )
                                      : fx_shr( (uint64_t)fpp, -2 * k ) < (uint64_t)fqq;
             int zb;
-            uint64_t const bm = fx_normal( fpq, zb );
-            FxRotation const r = fx_rotation( swap ? fqq : fpp, swap ? fpp : fqq, bm, zb, fpq.d[0] < 0,
-                                              swap ? dq : dp, swap ? dp : dq );
+            bool negative;
+            uint64_t const bm = fx_normal( fpq, zb, negative );
+            FxRotation const r = fx_rotation( swap ? fqq : fpp, swap ? fpp : fqq, bm, zb, negative, swap ? dq : dp,
+                                              swap ? dp : dq );
             bool fits = true;
             st.for_parts( [&]( int h ) {
-                // the rows' other columns j = 0, 1, ... past p and q, every
-                // second one: all loads first
+                // the rows' other columns, every second one: all loads first
                 constexpr int N = Lay::HALF - 1;
                 FxNum<3> fl[N], fs[N];
                 int up[N], uq[N];
 #pragma unroll
                 for ( int t = 0; t < N; ++t )
                 {
-                    int j = 2 * t + h;
-                    j += j >= p;
-                    j += j >= q;
-                    up[t] = Lay::pair( p, j );
-                    uq[t] = Lay::pair( q, j );
+                    st.column( u, p, q, 2 * t + h, up[t], uq[t] );
                     fl[t] = st.f( swap ? uq[t] : up[t] );
                     fs[t] = st.f( swap ? up[t] : uq[t] );
                 }
@@ -661,8 +691,9 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
             if ( ok && !fx_zero( v ) )
             {
                 int z;
-                uint64_t const m = fx_normal( v, z );
-                w = fx_double( m, d - d0 - z - FX_V, v.d[0] < 0 ) / fx_double( (uint64_t)f, 2 * d - FX_ONE, false );
+                bool negative;
+                uint64_t const m = fx_normal( v, z, negative );
+                w = fx_double( m, d - d0 - z - FX_V, negative ) / fx_double( (uint64_t)f, 2 * d - FX_ONE, false );
             }
             st.w( k ) = w;
         }

@@ -9,9 +9,10 @@
 // are the 35 distinct sums of monomials up to degree 4 (not 55 products), the
 // weight's quotient takes 3 operations, and the second pass reads the weights
 // the first one left in the coefficient array.  What is left is issue and
-// latency: about 2.6k warp instructions a rotation at 52% of the issue slots
-// with 10 warps an SM (shared memory), FP64 pipe 25%, ALU 44%.  2M quadratic
-// targets, k = 32: 84 -> 41 ms; 10k, k = 20: 1.20 -> 0.63 ms; 200k rows of 120
+// latency: about 2.4k warp instructions a rotation at 53% of the issue slots
+// with 10 warps an SM (shared memory), FP64 pipe 27%, ALU 37%.  The loop's code
+// is kept small: with its two halves unrolled the 2M setup takes 44 ms in place
+// of 37.6 (instruction fetch).  2M quadratic targets, k = 32: 84 -> 37.6 ms; 10k, k = 20: 1.20 -> 0.60 ms; 200k rows of 120
 // within a radius: 18.6 -> 8.9 ms; the batched setup of 1.5M targets 26 -> 15.
 //
 // Targets the fixed-point form hands back (near-singular moments, scales out
@@ -168,6 +169,11 @@ template <int M>
 struct FixedLayout
 {
     static constexpr int OFF = M * ( M - 1 ) / 2;
+    // a block's table of FxLayout::column: (up, uq) of pair u and index t as two
+    // bytes at u * PITCH + t (the odd pitch spreads the lanes' rows over the
+    // banks)
+    static constexpr int PITCH = M > 2 ? ( M - 2 ) | 1 : 1;
+    static constexpr size_t TABLE = ( OFF * PITCH * sizeof( uint16_t ) + 15 ) / 16 * 16;
     // bytes a matrix
     static constexpr size_t BYTES =
         ( OFF + 2 * M ) * sizeof( int2 ) + OFF * sizeof( int32_t ) + ( M + 3 ) / 4 * 4;
@@ -180,13 +186,16 @@ struct FixedState
     int2 *N;    // leading digits of F, its diagonal, V
     int32_t *L; // last digits of F
     int8_t *E;
+    uint16_t const *T;
     double *W;
     int64_t ut, us;
     int part;
-    __device__ FixedState( void *warp_smem, int lane, double *work, int64_t warp, int64_t warps )
+    __device__ FixedState( void *warp_smem, uint16_t const *table, int lane, double *work, int64_t warp,
+                           int64_t warps )
         : N( (int2 *)warp_smem + lane % COLS )
         , L( (int32_t *)( (int2 *)warp_smem + ( OFF + 2 * M ) * COLS ) + lane % COLS )
         , E( (int8_t *)( (int32_t *)( (int2 *)warp_smem + ( OFF + 2 * M ) * COLS ) + OFF * COLS ) + lane % COLS )
+        , T( table )
         , W( work )
         , ut( warp * COLS + lane % COLS )
         , us( warps * COLS )
@@ -222,6 +231,12 @@ struct FixedState
         N[( OFF + M + k ) * COLS] = make_int2( x.d[0], x.d[1] );
     }
     __device__ __forceinline__ double &w( int k ) const { return a( OFF + M + k ); }
+    __device__ __forceinline__ void column( int u, int, int, int t, int &up, int &uq ) const
+    {
+        int const x = T[u * FixedLayout<M>::PITCH + t];
+        up = x & 255;
+        uq = x >> 8;
+    }
     __device__ __forceinline__ int exp( int k ) const { return E[k * COLS]; }
     __device__ __forceinline__ void set_exp( int k, int d ) const { E[k * COLS] = (int8_t)d; }
     __device__ __forceinline__ double2 &rot( int r ) const { return reinterpret_cast<double2 *>( W )[r * us + ut]; }
@@ -270,6 +285,24 @@ struct FixedState
         return ( m & ( m >> 16 | m << 16 ) ) >> ( threadIdx.x & 31 ) & 1u;
     }
 };
+
+// Fills a block's table (all its threads; a barrier follows).
+template <int M>
+__device__ __forceinline__ void fill_columns( uint16_t *table )
+{
+    if constexpr ( M > 2 )
+    {
+        using Lay = FxLayout<M>;
+        for ( int x = threadIdx.x; x < Lay::OFF * ( M - 2 ); x += blockDim.x )
+        {
+            int p, q, up, uq;
+            Lay::of_slot( x / ( M - 2 ), p, q );
+            Lay::column( p, q, x % ( M - 2 ), up, uq );
+            table[x / ( M - 2 ) * FixedLayout<M>::PITCH + x % ( M - 2 )] = (uint16_t)( up | uq << 8 );
+        }
+    }
+}
+
 constexpr int FX_WORK = 2 * FX_LOG + FX_LOG / 8; // doubles of the log a matrix
 
 // Row 0 of the pseudo-inverse from the moments in the state's entries (as
@@ -563,8 +596,11 @@ __global__ void __launch_bounds__( 32 * FIXED_WARPS<COLS>, FIXED_BLOCKS_PER_SM<C
     int const lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     int64_t const warp = blockIdx.x * (int64_t)FIXED_WARPS<COLS> + wib,
                   warps = gridDim.x * (int64_t)FIXED_WARPS<COLS>;
-    void *const wsm = (char *)smem + wib * FixedLayout<M>::BYTES * COLS;
-    FixedState<M, COLS> const st( wsm, lane, work, warp, warps );
+    uint16_t *const table = (uint16_t *)smem;
+    fill_columns<M>( table );
+    __syncthreads();
+    void *const wsm = (char *)smem + FixedLayout<M>::TABLE + wib * FixedLayout<M>::BYTES * COLS;
+    FixedState<M, COLS> const st( wsm, table, lane, work, warp, warps );
     unsigned iters = 0;
     for ( int64_t g = warp * COLS; g < n_tgt; g += warps * COLS )
     {
@@ -579,10 +615,10 @@ __global__ void __launch_bounds__( 32 * FIXED_WARPS<COLS>, FIXED_BLOCKS_PER_SM<C
 
 // One task of a batch: up to 32 targets of one bucket.
 template <int M>
-__device__ void fixed_task( BatchSetupArgs const &a, SetupTask const &t, int rbf, int G, void *wsm, int64_t warp,
-                            int64_t warps, int cap, unsigned &iters, int lane )
+__device__ void fixed_task( BatchSetupArgs const &a, SetupTask const &t, int rbf, int G, void *wsm,
+                            uint16_t const *table, int64_t warp, int64_t warps, int cap, unsigned &iters, int lane )
 {
-    FixedState<M, 32> const st( wsm, lane, a.u_work, warp, warps );
+    FixedState<M, 32> const st( wsm, table, lane, a.u_work, warp, warps );
     unsigned rest = FULL >> ( 32 - t.count );
     if ( fixed_supported( rbf ) )
         rest = fixed_targets<M, 32>( a.nb, a.tgt, a.offset, a.list, t.first, t.count, rbf, G, a.rows_sorted,
@@ -613,7 +649,12 @@ __global__ void __launch_bounds__( 32 * FIXED_WARPS<32>, FIXED_BLOCKS_PER_SM<32>
     extern __shared__ double smem[];
     int const lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     int64_t const warp = blockIdx.x * (int64_t)FIXED_WARPS<32> + wib, warps = gridDim.x * (int64_t)FIXED_WARPS<32>;
-    void *const wsm = (char *)smem + wib * FixedLayout<10>::BYTES * 32;
+    uint16_t *const table10 = (uint16_t *)smem, *const table4 = table10 + FixedLayout<10>::TABLE / sizeof( uint16_t );
+    fill_columns<10>( table10 );
+    fill_columns<4>( table4 );
+    __syncthreads();
+    void *const wsm =
+        (char *)smem + FixedLayout<10>::TABLE + FixedLayout<4>::TABLE + wib * FixedLayout<10>::BYTES * 32;
     int64_t const t_end = a.t_end >= 0 ? a.t_end : *a.n_tasks;
     unsigned iters = 0;
     for ( ;; )
@@ -638,11 +679,11 @@ __global__ void __launch_bounds__( 32 * FIXED_WARPS<32>, FIXED_BLOCKS_PER_SM<32>
         }
         int const cap = (int)min( a.jcap[basis], (unsigned)FX_LOG );
         if ( basis == DTK_CONSTANT3 )
-            fixed_task<1>( a, t, rbf, G, wsm, warp, warps, cap, iters, lane );
+            fixed_task<1>( a, t, rbf, G, wsm, nullptr, warp, warps, cap, iters, lane );
         else if ( basis == DTK_LINEAR3 )
-            fixed_task<4>( a, t, rbf, G, wsm, warp, warps, cap, iters, lane );
+            fixed_task<4>( a, t, rbf, G, wsm, table4, warp, warps, cap, iters, lane );
         else
-            fixed_task<10>( a, t, rbf, G, wsm, warp, warps, cap, iters, lane );
+            fixed_task<10>( a, t, rbf, G, wsm, table10, warp, warps, cap, iters, lane );
     }
     add_rotations( iters, a.rotations );
 }
@@ -665,7 +706,7 @@ unsigned fixed_blocks( int64_t n )
 template <int M, int COLS>
 void launch_fixed( SetupArgs const &a, double *work, uint32_t *list, unsigned *count, cudaStream_t s )
 {
-    size_t const smem = FixedLayout<M>::BYTES * COLS * FIXED_WARPS<COLS>;
+    size_t const smem = FixedLayout<M>::TABLE + FixedLayout<M>::BYTES * COLS * FIXED_WARPS<COLS>;
     ensure_dynamic_smem( k_setup_fixed<M, COLS>, smem );
     Neighbours const nb{a.src, a.idx, a.pos, a.s2};
     int const cap = (int)std::min<unsigned long long>( jacobi_cap( M ), FX_LOG );
@@ -720,7 +761,8 @@ void setup_fixed( SetupArgs const &a, double *work, uint32_t *list, unsigned *co
 
 void batch_fixed( BatchSetupArgs const &a, cudaStream_t s )
 {
-    size_t const smem = FixedLayout<10>::BYTES * 32 * FIXED_WARPS<32>;
+    size_t const smem =
+        FixedLayout<10>::TABLE + FixedLayout<4>::TABLE + FixedLayout<10>::BYTES * 32 * FIXED_WARPS<32>;
     ensure_dynamic_smem( k_batch_fixed, smem );
     k_batch_fixed<<<(unsigned)( FIXED_BLOCKS_PER_SM<32> * num_sms() ), 32 * FIXED_WARPS<32>, smem, s>>>( a );
     check_launch( "k_batch_fixed" );

@@ -55,6 +55,7 @@ struct State
     }
     void set_v( int k, FxNum<2> const &x ) const { std::memcpy( &vw[k], x.d, 8 ); }
     double &w( int k ) const { return vw[k]; }
+    void column( int, int p, int q, int t, int &up, int &uq ) const { Lay::column( p, q, t, up, uq ); }
     int exp( int k ) const { return e[k]; }
     void set_exp( int k, int d ) const { e[k] = d; }
     void log( int r, double c_, double s_, int l ) const
