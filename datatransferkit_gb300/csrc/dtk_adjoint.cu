@@ -13,9 +13,12 @@
 //                 - [j farthest] 1.1 (sum_l g_l rho^_l) / R u_j
 //     with alpha_j = a^.P^_j, e_j = v_j - P^_j.z^, g_j = alpha_j e_j rbf'(rho^_j),
 //     u_j = x_j / rho_j; the radius max sends its gradient to the farthest
-//     neighbour (the last of largest rho in row order).  The per-entry
-//     contributions cot_i dy/dx_j are written once and gathered through the
-//     same transpose.  The pseudo-inverse is recomputed per target (never
+//     neighbour (the last of largest rho in row order): the only term that
+//     needs the sum over the row, so one pass writes every entry's contribution
+//     and the farthest one is corrected after it.  The contributions cot_i
+//     dy/dx_j, with c_j cot_i beside them, are written at the entry's place in
+//     the transpose (one 32-byte sector each), so each source sums a run of
+//     consecutive sectors.  The pseudo-inverse is recomputed per target (never
 //     stored) from FP64 scaled moments.  Well-conditioned targets take an
 //     FP64 Cholesky (A^+ = A^-1 there); the rest take an FP32 round-robin
 //     Jacobi, one FP64 sweep on B = V32^T A V32 and truncation at 2^-40 of
@@ -24,6 +27,7 @@
 #include "dtk_common.cuh"
 #include "dtk_handle.cuh"
 #include "dtk_jacobi.cuh"
+#include "dtk_moments.cuh"
 
 #include <algorithm>
 #include <new>
@@ -67,65 +71,84 @@ __global__ void k_entry_rows( int32_t const *offset, int64_t n_tgt, int32_t *row
             row_of[e] = (int32_t)i;
 }
 
-// One thread per source: grad_values[s] = sum_e coeff[e] cot[row(e)] and
-// grad_coords[s] = sum_e contrib[e] over the source's entries, ascending.
+// t_place[e] = the place of entry e in the transpose
+__global__ void k_entry_places( int32_t const *t_entry, int64_t nnz, int32_t *t_place )
+{
+    int64_t const q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if ( q < nnz )
+        t_place[t_entry[q]] = (int32_t)q;
+}
+
+// One thread per source: grad_values[s] = sum_e coeff[e] cot[row(e)] over the
+// source's entries, ascending.
 template <bool F32>
 __global__ void k_transpose_gather( int64_t n_src, int32_t const *t_offset, int32_t const *t_entry,
                                     int uniform_row, int32_t const *row_of, void const *coeff,
-                                    double const *cot, double const *contrib, double *grad_values,
-                                    double *grad_coords )
+                                    double const *cot, double *grad_values )
 {
     int64_t const s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if ( s >= n_src )
         return;
-    double gv = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+    double gv = 0.0;
     for ( int q = t_offset[s]; q < t_offset[s + 1]; ++q )
     {
         int64_t const e = t_entry[q];
         int64_t const row = uniform_row > 0 ? e / uniform_row : row_of[e];
         double const c = F32 ? (double)static_cast<float const *>( coeff )[e]
                              : static_cast<double const *>( coeff )[e];
-        gv = fma( c, cot[row], gv );
-        if ( contrib )
-        {
-            gx += contrib[3 * e + 0];
-            gy += contrib[3 * e + 1];
-            gz += contrib[3 * e + 2];
-        }
+        gv = __dadd_rn( gv, __dmul_rn( c, cot[row] ) );
     }
     grad_values[s] = gv;
-    if ( grad_coords )
-    {
-        grad_coords[3 * s + 0] = gx;
-        grad_coords[3 * s + 1] = gy;
-        grad_coords[3 * s + 2] = gz;
-    }
 }
 
-// Jacobian of the scaled basis: row c of dP/dx^ at x^ (3 entries).
-template <int M>
-__device__ __forceinline__ void basis_jac_row( int c, double x, double y, double z, double *g )
+// The same sums and those of the coordinates from the entries' contributions,
+// which lie in the transpose's order (x, y, z, value: 32 bytes an entry): four
+// lanes a source, one a component, so that a warp reads whole lines.  1M x 1M,
+// k = 32: 1.47 ms as gathers through the entries' indices (three cache lines an
+// entry).
+__global__ void k_transpose_sum( int64_t n_src, int32_t const *t_offset, double const *contrib, double *grad_values,
+                                 double *grad_coords )
 {
-    g[0] = g[1] = g[2] = 0.0;
-    if constexpr ( M >= 4 )
-    {
-        if ( c >= 1 && c <= 3 )
-            g[c - 1] = 1.0;
-    }
-    if constexpr ( M == 10 )
-    {
-        switch ( c )
-        {
-        case 4: g[0] = 2.0 * x; break;
-        case 5: g[0] = y; g[1] = x; break;
-        case 6: g[0] = z; g[2] = x; break;
-        case 7: g[1] = 2.0 * y; break;
-        case 8: g[1] = z; g[2] = y; break;
-        case 9: g[2] = 2.0 * z; break;
-        default: break;
-        }
-    }
+    int64_t const t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int64_t const s = t >> 2;
+    int const c = (int)( t & 3 );
+    if ( s >= n_src )
+        return;
+    int64_t const b = t_offset[s], e = t_offset[s + 1];
+    double sum = 0.0;
+#pragma unroll 4
+    for ( int64_t q = b; q < e; ++q )
+        sum = __dadd_rn( sum, __ldcs( contrib + 4 * q + c ) );
+    if ( c == 3 )
+        grad_values[s] = sum;
+    else
+        grad_coords[3 * s + c] = sum;
 }
+
+// What the coordinate-adjoint kernels read and write.
+struct AdjointView
+{
+    double const *src, *tgt;
+    int32_t const *offset, *idx, *place; // place: of each entry in the transpose
+    int64_t n_src;
+    int rbf;
+    double const *values, *cot;
+    double const *coeff64;
+    float const *coeff32;
+    double *contrib; // 4 doubles an entry, in the transpose's order
+    unsigned *status;
+    __device__ __forceinline__ void put( int64_t e, double x, double y, double z, double value ) const
+    {
+        double2 *const p = reinterpret_cast<double2 *>( contrib + 4 * (int64_t)place[e] );
+        p[0] = make_double2( x, y );
+        p[1] = make_double2( z, value );
+    }
+    // the entry's part of grad_values
+    __device__ __forceinline__ double value( int64_t e, double ci ) const
+    {
+        return __dmul_rn( coeff32 ? (double)coeff32[e] : coeff64[e], ci );
+    }
+};
 
 // Per-target pieces shared by the two coordinate-adjoint kernels.
 struct AdjTarget
@@ -138,152 +161,209 @@ struct AdjTarget
 
 // Returns false when the target needs no more work (no entries, a zero
 // cotangent: its contributions are zero, or a bad index: reported).
-__device__ __forceinline__ bool adjoint_prologue( int64_t i, double const *src, double const *tgt,
-                                                 int32_t const *offset, int32_t const *idx, int64_t n_src,
-                                                 double const *cot, double *contrib, unsigned *status,
-                                                 AdjTarget &T )
+__device__ __forceinline__ bool adjoint_prologue( int64_t i, AdjointView const &v, AdjTarget &T )
 {
     T.i = i;
-    T.b0 = offset[i];
-    T.len = offset[i + 1] - (int)T.b0;
-    T.ci = cot[i];
+    T.b0 = v.offset[i];
+    T.len = v.offset[i + 1] - (int)T.b0;
+    T.ci = v.cot[i];
     if ( T.len == 0 )
         return false;
     for ( int j = 0; j < T.len; ++j )
-        if ( (uint32_t)idx[T.b0 + j] >= (uint64_t)n_src )
+        if ( (uint32_t)v.idx[T.b0 + j] >= (uint64_t)v.n_src )
         {
-            atomicOr( status, DEV_BAD_INDEX );
+            atomicOr( v.status, DEV_BAD_INDEX );
             return false;
         }
     if ( T.ci == 0.0 )
     {
         for ( int j = 0; j < T.len; ++j )
-            contrib[3 * ( T.b0 + j )] = contrib[3 * ( T.b0 + j ) + 1] = contrib[3 * ( T.b0 + j ) + 2] = 0.0;
+            v.put( T.b0 + j, 0.0, 0.0, 0.0, v.value( T.b0 + j, T.ci ) );
         return false;
     }
-    T.tx = tgt[3 * i];
-    T.ty = tgt[3 * i + 1];
-    T.tz = tgt[3 * i + 2];
+    T.tx = v.tgt[3 * i];
+    T.ty = v.tgt[3 * i + 1];
+    T.tz = v.tgt[3 * i + 2];
     // radius and the farthest neighbour (last of largest distance)
-    double dmax = 0.0;
+    double d2max = 0.0;
     T.far = 0;
     for ( int j = 0; j < T.len; ++j )
     {
-        int64_t const sj = idx[T.b0 + j];
-        double const x = src[3 * sj] - T.tx, y = src[3 * sj + 1] - T.ty, z = src[3 * sj + 2] - T.tz;
-        double const d = sqrt( ( x * x + y * y ) + z * z );
-        if ( d >= dmax )
+        int64_t const sj = v.idx[T.b0 + j];
+        double const d2 = dist2_rn( v.src[3 * sj], v.src[3 * sj + 1], v.src[3 * sj + 2], T.tx, T.ty, T.tz );
+        if ( d2 >= d2max )
         {
-            dmax = d;
+            d2max = d2;
             T.far = j;
         }
     }
-    double const floor_d = 10. * DBL_EPSILON;
+    double const floor_d = 10. * DBL_EPSILON, dmax = sqrt( d2max );
     T.radius_live = dmax > floor_d;
     T.inv_r = 1.0 / ( 1.1 * ( T.radius_live ? dmax : floor_d ) );
     return true;
 }
 
-// Scaled moments A^ (upper triangle) and b^ = sum phi v P^ (FP64).
-template <int M>
-__device__ __forceinline__ void adjoint_moments( AdjTarget const &T, double const *src, int32_t const *idx,
-                                                 int rbf, double const *values, double *A, double *bh )
+// An entry's scaled coordinates, their squares, 1 / |x^| (0 at the target) and
+// |x^|: one reciprocal square root.
+struct AdjEntry
 {
-    constexpr int NU = M * ( M + 1 ) / 2;
+    int64_t sj;
+    double x, y, z, xx, yy, zz, inv_rho, rho;
+};
+__device__ __forceinline__ AdjEntry adjoint_entry( AdjTarget const &T, AdjointView const &v, int j )
+{
+    AdjEntry a;
+    a.sj = v.idx[T.b0 + j];
+    a.x = ( v.src[3 * a.sj] - T.tx ) * T.inv_r;
+    a.y = ( v.src[3 * a.sj + 1] - T.ty ) * T.inv_r;
+    a.z = ( v.src[3 * a.sj + 2] - T.tz ) * T.inv_r;
+    a.xx = a.x * a.x;
+    a.yy = a.y * a.y;
+    a.zz = a.z * a.z;
+    double const d2 = ( a.xx + a.yy ) + a.zz;
+    a.inv_rho = d2 > 0.0 ? rsqrt( d2 ) : 0.0;
+    a.rho = d2 * a.inv_rho;
+    return a;
+}
+
+// rbf(x) and rbf'(x); the common Wendland functions share their powers.
+__device__ __forceinline__ void rbf_with_deriv( int rbf, double x, double &phi, double &deriv )
+{
+    double const y = 1.0 - x, y2 = y * y, y3 = y2 * y;
+    if ( rbf == DTK_WENDLAND2 )
+    {
+        phi = y2 * y2 * fma( 4.0, x, 1.0 );
+        deriv = -20.0 * x * y3;
+    }
+    else if ( rbf == DTK_WENDLAND4 )
+    {
+        phi = y3 * y3 * fma( fma( 35.0, x, 18.0 ), x, 3.0 );
+        deriv = -56.0 * x * fma( 5.0, x, 1.0 ) * ( y3 * y2 );
+    }
+    else
+    {
+        phi = rbf_eval<double>( rbf, x );
+        deriv = rbf_deriv( rbf, x );
+    }
+}
+
+// Scaled moments A^ (upper triangle) and b^ = sum phi v P^ (FP64).  The
+// quadratic basis has 35 distinct sums for its 55 entries.
+template <int M>
+__device__ __forceinline__ void adjoint_moments( AdjTarget const &T, AdjointView const &v, double *A, double *bh )
+{
+    double S[N_MOMENTS<M>];
 #pragma unroll
-    for ( int u = 0; u < NU; ++u )
-        A[u] = 0.0;
+    for ( int u = 0; u < N_MOMENTS<M>; ++u )
+        S[u] = 0.0;
 #pragma unroll
     for ( int c = 0; c < M; ++c )
         bh[c] = 0.0;
     for ( int j = 0; j < T.len; ++j )
     {
-        int64_t const sj = idx[T.b0 + j];
-        double const x = ( src[3 * sj] - T.tx ) * T.inv_r, y = ( src[3 * sj + 1] - T.ty ) * T.inv_r,
-                     z = ( src[3 * sj + 2] - T.tz ) * T.inv_r;
+        AdjEntry const a = adjoint_entry( T, v, j );
+        double const phi = rbf_eval<double>( v.rbf, a.rho );
         double P[M];
-        basis_eval<M, double>( x, y, z, P );
-        double const phi = rbf_eval<double>( rbf, sqrt( ( x * x + y * y ) + z * z ) );
-        double const pv = phi * values[sj];
+        basis_eval<M, double>( a.x, a.y, a.z, P );
+        double const pv = phi * v.values[a.sj];
 #pragma unroll
-        for ( int a = 0; a < M; ++a )
-        {
-            double const pa = phi * P[a];
-            bh[a] = fma( pv, P[a], bh[a] );
+        for ( int c = 0; c < M; ++c )
+            bh[c] = fma( pv, P[c], bh[c] );
+        add_moments<M>( a.x, a.y, a.z, a.xx, a.yy, a.zz, phi, S );
+    }
 #pragma unroll
-            for ( int c = a; c < M; ++c )
-                A[ut<M>( a, c )] = fma( pa, P[c], A[ut<M>( a, c )] );
-        }
+    for ( int a = 0; a < M; ++a )
+#pragma unroll
+        for ( int c = a; c < M; ++c )
+            A[ut<M>( a, c )] = S[moment_index( a, c )];
+}
+
+// P . a
+template <int M>
+__device__ __forceinline__ double adjoint_dot( double const *a, AdjEntry const &e )
+{
+    double r = a[0];
+    if constexpr ( M >= 4 )
+        r = fma( a[3], e.z, fma( a[2], e.y, fma( a[1], e.x, r ) ) );
+    if constexpr ( M == 10 )
+    {
+        r = fma( e.x, fma( a[4], e.x, fma( a[5], e.y, a[6] * e.z ) ), r );
+        r = fma( e.y, fma( a[7], e.y, a[8] * e.z ), r );
+        r = fma( a[9], e.zz, r );
+    }
+    return r;
+}
+
+// d(P . a) / dx^ : a2 = twice a[4], a[7], a[9]
+template <int M>
+__device__ __forceinline__ void adjoint_grad( double const *a, double const *a2, AdjEntry const &e, double *g )
+{
+    if constexpr ( M == 1 )
+        g[0] = g[1] = g[2] = 0.0;
+    else
+    {
+        g[0] = a[1];
+        g[1] = a[2];
+        g[2] = a[3];
+    }
+    if constexpr ( M == 10 )
+    {
+        g[0] = fma( a2[0], e.x, fma( a[5], e.y, fma( a[6], e.z, g[0] ) ) );
+        g[1] = fma( a[5], e.x, fma( a2[1], e.y, fma( a[8], e.z, g[1] ) ) );
+        g[2] = fma( a[6], e.x, fma( a[8], e.y, fma( a2[2], e.z, g[2] ) ) );
     }
 }
 
-// Given a^ = A^+ e0 and z^ = A^+ b^: pass 1, S = sum g_l rho^_l; pass 2, the
-// per-entry contributions cot_i dy/dx_j.
+// Given a^ = A^+ e0 and z^ = A^+ b^: the per-entry contributions cot_i dy/dx_j
+// and S = sum g_l rho^_l in one pass, then the radius term of the farthest
+// neighbour.
 template <int M>
-__device__ __forceinline__ void adjoint_passes( AdjTarget const &T, double const *src, int32_t const *idx,
-                                                int rbf, double const *values, double const *ah,
-                                                double const *zh, double *contrib )
+__device__ __forceinline__ void adjoint_passes( AdjTarget const &T, AdjointView const &v, double const *ah,
+                                                double const *zh )
 {
-    double S = 0.0;
-    for ( int j = 0; j < T.len; ++j )
+    double a2[3] = {0.0, 0.0, 0.0}, z2[3] = {0.0, 0.0, 0.0};
+    if constexpr ( M == 10 )
     {
-        int64_t const sj = idx[T.b0 + j];
-        double const x = ( src[3 * sj] - T.tx ) * T.inv_r, y = ( src[3 * sj + 1] - T.ty ) * T.inv_r,
-                     z = ( src[3 * sj + 2] - T.tz ) * T.inv_r;
-        double P[M];
-        basis_eval<M, double>( x, y, z, P );
-        double const rh = sqrt( ( x * x + y * y ) + z * z );
-        double al = 0.0, pz = 0.0;
-#pragma unroll
-        for ( int c = 0; c < M; ++c )
-        {
-            al = fma( ah[c], P[c], al );
-            pz = fma( P[c], zh[c], pz );
-        }
-        double const e = values[sj] - pz;
-        S = fma( al * e * rbf_deriv( rbf, rh ), rh, S );
+        a2[0] = 2.0 * ah[4];
+        a2[1] = 2.0 * ah[7];
+        a2[2] = 2.0 * ah[9];
+        z2[0] = 2.0 * zh[4];
+        z2[1] = 2.0 * zh[7];
+        z2[2] = 2.0 * zh[9];
     }
+    double const scale = T.ci * T.inv_r;
+    double S = 0.0, fx = 0.0, fy = 0.0, fz = 0.0, ux = 0.0, uy = 0.0, uz = 0.0;
     for ( int j = 0; j < T.len; ++j )
     {
-        int64_t const sj = idx[T.b0 + j];
-        double x = src[3 * sj] - T.tx, y = src[3 * sj + 1] - T.ty, z = src[3 * sj + 2] - T.tz;
-        double const rho = sqrt( ( x * x + y * y ) + z * z );
-        double const ux = rho > 0.0 ? x / rho : 0.0, uy = rho > 0.0 ? y / rho : 0.0,
-                     uz = rho > 0.0 ? z / rho : 0.0;
-        x *= T.inv_r;
-        y *= T.inv_r;
-        z *= T.inv_r;
-        double P[M];
-        basis_eval<M, double>( x, y, z, P );
-        double const rh = sqrt( ( x * x + y * y ) + z * z );
-        double const phi = rbf_eval<double>( rbf, rh );
-        double al = 0.0, pz = 0.0;
-#pragma unroll
-        for ( int c = 0; c < M; ++c )
+        AdjEntry const a = adjoint_entry( T, v, j );
+        double phi, deriv;
+        rbf_with_deriv( v.rbf, a.rho, phi, deriv );
+        double const al = adjoint_dot<M>( ah, a ), e = v.values[a.sj] - adjoint_dot<M>( zh, a );
+        double ga[3], gz[3];
+        adjoint_grad<M>( ah, a2, a, ga );
+        adjoint_grad<M>( zh, z2, a, gz );
+        double const g = al * e * deriv;
+        S = fma( g, a.rho, S );
+        // phi (e grad(P . a) - al grad(P . z)) + g u, u = x^ / rho^
+        double const pe = phi * e, pa = phi * al, gr = g * a.inv_rho;
+        double const cx = scale * fma( gr, a.x, fma( pe, ga[0], -( pa * gz[0] ) ) ),
+                     cy = scale * fma( gr, a.y, fma( pe, ga[1], -( pa * gz[1] ) ) ),
+                     cz = scale * fma( gr, a.z, fma( pe, ga[2], -( pa * gz[2] ) ) );
+        v.put( T.b0 + j, cx, cy, cz, v.value( T.b0 + j, T.ci ) );
+        if ( j == T.far )
         {
-            al = fma( ah[c], P[c], al );
-            pz = fma( P[c], zh[c], pz );
+            fx = cx;
+            fy = cy;
+            fz = cz;
+            ux = a.x * a.inv_rho;
+            uy = a.y * a.inv_rho;
+            uz = a.z * a.inv_rho;
         }
-        double const e = values[sj] - pz;
-        double const gj = al * e * rbf_deriv( rbf, rh );
-        double G[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for ( int c = 1; c < M; ++c )
-        {
-            double jr[3];
-            basis_jac_row<M>( c, x, y, z, jr );
-            double const w = e * ah[c] - al * zh[c];
-            G[0] = fma( w, jr[0], G[0] );
-            G[1] = fma( w, jr[1], G[1] );
-            G[2] = fma( w, jr[2], G[2] );
-        }
-        double coef = gj;
-        if ( j == T.far && T.radius_live )
-            coef -= 1.1 * S;
-        double const sp = phi * T.inv_r, sc = coef * T.inv_r;
-        contrib[3 * ( T.b0 + j ) + 0] = T.ci * ( sp * G[0] + sc * ux );
-        contrib[3 * ( T.b0 + j ) + 1] = T.ci * ( sp * G[1] + sc * uy );
-        contrib[3 * ( T.b0 + j ) + 2] = T.ci * ( sp * G[2] + sc * uz );
+    }
+    if ( T.radius_live )
+    {
+        double const r = -1.1 * S * scale;
+        v.put( T.b0 + T.far, fma( r, ux, fx ), fma( r, uy, fy ), fma( r, uz, fz ), v.value( T.b0 + T.far, T.ci ) );
     }
 }
 
@@ -298,9 +378,7 @@ constexpr int AF = 32; // threads per block of the fast kernel
 
 template <int M>
 __global__ void __launch_bounds__( AF )
-    k_adjoint_fast( double const *src, double const *tgt, int32_t const *offset, int32_t const *idx,
-                    uint32_t const *order, int64_t n_tgt, int64_t n_src, int rbf, double const *values,
-                    double const *cot, double *contrib, int32_t *list, unsigned *count, unsigned *status )
+    k_adjoint_fast( AdjointView v, uint32_t const *order, int64_t n_tgt, int32_t *list, unsigned *count )
 {
     constexpr int NU = M * ( M + 1 ) / 2;
     // per thread, interleaved: NU moments, M of b^, NU of the Cholesky work area
@@ -311,12 +389,12 @@ __global__ void __launch_bounds__( AF )
         return;
     int64_t const i = order ? (int64_t)order[g] : g;
     AdjTarget T;
-    if ( !adjoint_prologue( i, src, tgt, offset, idx, n_src, cot, contrib, status, T ) )
+    if ( !adjoint_prologue( i, v, T ) )
         return;
     double A[NU];
     {
         double bh[M];
-        adjoint_moments<M>( T, src, idx, rbf, values, A, bh );
+        adjoint_moments<M>( T, v, A, bh );
 #pragma unroll
         for ( int c = 0; c < M; ++c )
             s_mom[( NU + c ) * AF + threadIdx.x] = bh[c];
@@ -343,9 +421,8 @@ __global__ void __launch_bounds__( AF )
             for ( int k = 0; k < j; ++k )
                 d = fma( -Wk( ut<M>( k, j ) ), Wk( ut<M>( k, j ) ), d );
             ok = ok && d > 0.0;
-            double const r = d > 0.0 ? sqrt( d ) : 1.0;
-            rinv[j] = 1.0 / r;
-            Wk( ut<M>( j, j ) ) = r;
+            rinv[j] = d > 0.0 ? rsqrt( d ) : 1.0;
+            Wk( ut<M>( j, j ) ) = d > 0.0 ? d * rinv[j] : 1.0;
 #pragma unroll
             for ( int c = j + 1; c < M; ++c )
             {
@@ -427,7 +504,7 @@ __global__ void __launch_bounds__( AF )
     double ah[M], zh[M];
     solve( true, ah );
     solve( false, zh );
-    adjoint_passes<M>( T, src, idx, rbf, values, ah, zh, contrib );
+    adjoint_passes<M>( T, v, ah, zh );
 }
 
 // Eigen path over the targets the fast path listed (list[0 .. *count),
@@ -435,9 +512,7 @@ __global__ void __launch_bounds__( AF )
 // truncation at 2^-40 of the largest eigenvalue, one FP64 refinement step.
 template <int M>
 __global__ void __launch_bounds__( AB )
-    k_adjoint_entries( double const *src, double const *tgt, int32_t const *offset, int32_t const *idx,
-                       int32_t const *list, unsigned const *count, int64_t n_src, int rbf,
-                       double const *values, double const *cot, double *contrib, unsigned *status )
+    k_adjoint_entries( AdjointView v, int32_t const *list, unsigned const *count )
 {
     constexpr int NU = M * ( M + 1 ) / 2;
     extern __shared__ unsigned char smem_raw[];
@@ -458,12 +533,12 @@ __global__ void __launch_bounds__( AB )
     for ( int64_t g = blockIdx.x * (int64_t)AB + threadIdx.x; g < n_list; g += (int64_t)gridDim.x * AB )
     {
         AdjTarget T;
-        if ( !adjoint_prologue( list[g], src, tgt, offset, idx, n_src, cot, contrib, status, T ) )
+        if ( !adjoint_prologue( list[g], v, T ) )
             continue;
         double bh[M];
         {
             double A[NU];
-            adjoint_moments<M>( T, src, idx, rbf, values, A, bh );
+            adjoint_moments<M>( T, v, A, bh );
 #pragma unroll
             for ( int u = 0; u < NU; ++u )
             {
@@ -552,30 +627,26 @@ __global__ void __launch_bounds__( AB )
             e0[r] = r == 0 ? 1.0 : 0.0;
         solve( e0, ah );
         solve( bh, zh );
-        adjoint_passes<M>( T, src, idx, rbf, values, ah, zh, contrib );
+        adjoint_passes<M>( T, v, ah, zh );
     }
 }
 
 template <int M>
-void launch_adjoint_entries( dtk_mls_s const *h, double const *values, double const *cot,
-                             double *contrib, unsigned *status, cudaStream_t s )
+void launch_adjoint_entries( dtk_mls_s const *h, AdjointView const &v, cudaStream_t s )
 {
     constexpr int NU = M * ( M + 1 ) / 2;
     DeviceBuffer<int32_t> list( std::max<int64_t>( 1, h->n_tgt ), s );
     DeviceBuffer<unsigned> count( 1, s );
     DTK_CUDA_OR_THROW( cudaMemsetAsync( count.get(), 0, sizeof( unsigned ), s ) );
     k_adjoint_fast<M><<<(unsigned)( ( h->n_tgt + AF - 1 ) / AF ), AF, ( 2 * NU + M ) * sizeof( double ) * AF, s>>>(
-        h->src_copy.get(), h->tgt_copy.get(), h->offset.get(), h->idx.get(), h->order.get(), h->n_tgt, h->n_src,
-        h->opts.rbf, values, cot, contrib, list.get(), count.get(), status );
+        v, h->order.get(), h->n_tgt, list.get(), count.get() );
     check_launch( "k_adjoint_fast" );
     size_t const smem = ( 2 * NU * sizeof( double ) + M * M * sizeof( double ) +
                           M * M * sizeof( float ) ) * AB;
     ensure_dynamic_smem( k_adjoint_entries<M>, smem );
     int64_t const want = ( h->n_tgt + AB - 1 ) / AB;
     unsigned const blocks = (unsigned)std::max<int64_t>( 1, std::min<int64_t>( want, 4 * num_sms() ) );
-    k_adjoint_entries<M><<<blocks, AB, smem, s>>>( h->src_copy.get(), h->tgt_copy.get(), h->offset.get(),
-                                                    h->idx.get(), list.get(), count.get(), h->n_src,
-                                                    h->opts.rbf, values, cot, contrib, status );
+    k_adjoint_entries<M><<<blocks, AB, smem, s>>>( v, list.get(), count.get() );
     check_launch( "k_adjoint_entries" );
 }
 
@@ -609,6 +680,13 @@ void build_transpose_for( dtk_mls_s *h, cudaStream_t s )
     h->t_offset.allocate( n_src + 1, s );
     k_narrow<<<(unsigned)( ( n_src + 256 ) / 256 ), 256, 0, s>>>( offs.get(), h->t_offset.get(), n_src );
     check_launch( "k_narrow" );
+    if ( h->src_copy.get() && nnz )
+    {
+        // for the coordinate adjoint
+        h->t_place.allocate( nnz, s );
+        k_entry_places<<<blocks, 256, 0, s>>>( h->t_entry.get(), nnz, h->t_place.get() );
+        check_launch( "k_entry_places" );
+    }
 }
 
 } // namespace
@@ -643,44 +721,52 @@ extern "C" dtk_status dtk_mls_apply_adjoint( dtk_mls_handle h, const double *cot
         build_transpose_for( h, s );
         DeviceBuffer<unsigned> status( 1, s );
         DTK_CUDA_OR_THROW( cudaMemsetAsync( status.get(), 0, sizeof( unsigned ), s ) );
-        DeviceBuffer<int32_t> row_of;
-        if ( h->uniform_row <= 0 && h->nnz )
-        {
-            row_of.allocate( h->nnz, s );
-            k_entry_rows<<<(unsigned)( ( h->n_tgt + 255 ) / 256 ), 256, 0, s>>>( h->offset.get(), h->n_tgt,
-                                                                                 row_of.get() );
-            check_launch( "k_entry_rows" );
-        }
-        DeviceBuffer<double> contrib;
         if ( grad_coords && h->nnz )
         {
-            contrib.allocate( 3 * h->nnz, s );
+            DeviceBuffer<double> contrib( 4 * h->nnz, s );
+            AdjointView const v{h->src_copy.get(), h->tgt_copy.get(), h->offset.get(),  h->idx.get(),
+                                h->t_place.get(),  h->n_src,          h->opts.rbf,      source_values,
+                                cot,               h->coeff64.get(),  h->coeff32.get(), contrib.get(),
+                                status.get()};
             switch ( h->opts.basis )
             {
             case DTK_CONSTANT3:
-                launch_adjoint_entries<1>( h, source_values, cot, contrib.get(), status.get(), s );
+                launch_adjoint_entries<1>( h, v, s );
                 break;
             case DTK_LINEAR3:
-                launch_adjoint_entries<4>( h, source_values, cot, contrib.get(), status.get(), s );
+                launch_adjoint_entries<4>( h, v, s );
                 break;
             default:
-                launch_adjoint_entries<10>( h, source_values, cot, contrib.get(), status.get(), s );
+                launch_adjoint_entries<10>( h, v, s );
                 break;
             }
+            k_transpose_sum<<<(unsigned)( ( 4 * h->n_src + 255 ) / 256 ), 256, 0, s>>>(
+                h->n_src, h->t_offset.get(), contrib.get(), grad_values, grad_coords );
+            check_launch( "k_transpose_sum" );
         }
-        if ( h->n_src )
+        else if ( h->n_src )
         {
+            if ( grad_coords )
+                DTK_CUDA_OR_THROW( cudaMemsetAsync( grad_coords, 0, 3 * h->n_src * sizeof( double ), s ) );
+            DeviceBuffer<int32_t> row_of;
+            if ( h->uniform_row <= 0 && h->nnz )
+            {
+                row_of.allocate( h->nnz, s );
+                k_entry_rows<<<(unsigned)( ( h->n_tgt + 255 ) / 256 ), 256, 0, s>>>( h->offset.get(), h->n_tgt,
+                                                                                     row_of.get() );
+                check_launch( "k_entry_rows" );
+            }
             unsigned const blocks = (unsigned)( ( h->n_src + 255 ) / 256 );
             bool const f32 = h->coeff32.get() != nullptr;
             void const *coeff = f32 ? (void const *)h->coeff32.get() : (void const *)h->coeff64.get();
             if ( f32 )
-                k_transpose_gather<true><<<blocks, 256, 0, s>>>(
-                    h->n_src, h->t_offset.get(), h->t_entry.get(), h->uniform_row, row_of.get(), coeff,
-                    cot, contrib.get(), grad_values, grad_coords );
+                k_transpose_gather<true><<<blocks, 256, 0, s>>>( h->n_src, h->t_offset.get(), h->t_entry.get(),
+                                                                 h->uniform_row, row_of.get(), coeff, cot,
+                                                                 grad_values );
             else
-                k_transpose_gather<false><<<blocks, 256, 0, s>>>(
-                    h->n_src, h->t_offset.get(), h->t_entry.get(), h->uniform_row, row_of.get(), coeff,
-                    cot, contrib.get(), grad_values, grad_coords );
+                k_transpose_gather<false><<<blocks, 256, 0, s>>>( h->n_src, h->t_offset.get(), h->t_entry.get(),
+                                                                  h->uniform_row, row_of.get(), coeff, cot,
+                                                                  grad_values );
             check_launch( "k_transpose_gather" );
         }
         unsigned st = 0;

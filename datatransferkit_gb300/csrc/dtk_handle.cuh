@@ -32,7 +32,8 @@ struct dtk_mls_s
     dtk::DeviceBuffer<double> src_copy, tgt_copy; // packed n x 3 (keep_points)
     // transpose of the CSR (source -> its entries, ascending), built on the
     // first adjoint call
-    dtk::DeviceBuffer<int32_t> t_offset, t_entry;
+    // (t_place: each entry's place in it, for the coordinate adjoint)
+    dtk::DeviceBuffer<int32_t> t_offset, t_entry, t_place;
     int64_t underdetermined = 0;
     int64_t rotations = 0, rotations32 = 0;
     float search_ms = 0.f, setup_ms = 0.f;
@@ -40,6 +41,7 @@ struct dtk_mls_s
 
     ~dtk_mls_s()
     {
-        life.retire( offset, idx, coeff64, coeff32, order, pos, perm, src_copy, tgt_copy, t_offset, t_entry );
+        life.retire( offset, idx, coeff64, coeff32, order, pos, perm, src_copy, tgt_copy, t_offset, t_entry,
+                     t_place );
     }
 };
