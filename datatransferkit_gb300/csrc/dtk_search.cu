@@ -1581,6 +1581,188 @@ __global__ void __launch_bounds__( Q_WARPS * 32, KNN_BLOCKS_PER_SM )
     }
 }
 
+// The nearest source (k = 1), one query a thread in the queries' Morton order.
+//
+// A list of one needs no warp: a lane keeps its two smallest FP32 squared
+// distances, and one threshold serves boxes and points alike, because a box's
+// nearest point is a point whose coordinates carry no more error than a
+// source's.  Every source whose key could be the least has d2_f <= T for
+// T = screen_threshold(U), U an upper bound of the least key from the smallest
+// d2_f seen.  When the second smallest exceeds T the smallest is the answer,
+// with no FP64 distance at all; otherwise (ties, near ties, coordinates whose
+// squares leave FP32's range) a second pass takes the exact FP64 key of every
+// source at or below T.
+//
+// The tree is walked depth first, nearest child first; the stack holds a node
+// and the children still open a level, so it is as deep as the tree.  Bound by
+// the latency of the dependent node loads: 2M queries over 2M sources in 1.04
+// ms, against 3.1 ms with a warp a query (exact FP64 seeds and a sorted list).
+constexpr int NN_THREADS = 128;
+constexpr int NN_BLOCKS_PER_SM = 8;
+constexpr int NN_LEVELS = 24; // deepest tree (levels below the root) the stack takes
+
+// U (see above) from the smallest d2_f: d2_f + spread (as d2_bounds, the axis
+// sum by Cauchy-Schwarz) rounded up, and 2^-140 for results below the normal
+// range; then the threshold.
+__device__ __forceinline__ float nearest_threshold( float d2, float err )
+{
+    float const root = __fmaf_ru( 7.f, __fsqrt_ru( d2 ), __fmul_ru( 3.f, err ) );
+    float const rel = __fmaf_ru( d2, 1.0f + 1.9073486328125e-06f, 7.1746481e-43f ); // 1 + 2^-19, 2^-140
+    return screen_threshold( __fmaf_ru( err, root, rel ), err );
+}
+
+__global__ void __launch_bounds__( NN_THREADS, NN_BLOCKS_PER_SM )
+    k_nearest( TreeView tr, PointsView tgt, uint32_t const *order, int32_t *idx_out, int32_t *pos_out,
+               unsigned *status )
+{
+    int64_t const w = blockIdx.x * (int64_t)NN_THREADS + threadIdx.x;
+    if ( w >= tgt.n )
+        return;
+    float const inf = __int_as_float( 0x7f800000 );
+    int const qi = order ? (int)order[w] : (int)w;
+    Query const q = make_query( tr.scene, tgt, qi );
+    float const tx = q.tf[0], ty = q.tf[1], tz = q.tf[2];
+    float T = inf, d_min = inf, d_next = inf;
+    int p_min = -1;
+    bool exact = false;
+    unsigned long long kd = KEY_INF;
+    int ki = 0x7fffffff, kp = -1;
+
+    auto dist2 = [&]( int p ) {
+        float4 const f = __ldg( tr.f4 + p );
+        float const dx = f.x - tx, dy = f.y - ty, dz = f.z - tz;
+        return fmaf( dz, dz, fmaf( dy, dy, dx * dx ) );
+    };
+    auto scan = [&]( int start, int end ) {
+        if ( exact )
+        {
+            for ( int p = start; p < end; ++p )
+                if ( !( dist2( p ) > T ) )
+                {
+                    double2 const e = sorted_dist2( tr, p, q );
+                    unsigned long long const d = (unsigned long long)__double_as_longlong( e.x );
+                    int const i = (int)__double_as_longlong( e.y );
+                    if ( key_less( d, i, kd, ki ) )
+                    {
+                        kd = d;
+                        ki = i;
+                        kp = p;
+                    }
+                }
+            return;
+        }
+        for ( int p = start; p < end; p += 4 )
+        {
+            float d[4];
+#pragma unroll
+            for ( int j = 0; j < 4; ++j )
+                d[j] = p + j < end ? dist2( p + j ) : inf;
+#pragma unroll
+            for ( int j = 0; j < 4; ++j )
+            {
+                d_next = fminf( d_next, fmaxf( d_min, d[j] ) );
+                p_min = d[j] < d_min ? p + j : p_min;
+                d_min = fminf( d_min, d[j] );
+            }
+        }
+        T = nearest_threshold( d_min, q.err );
+    };
+    // squared distance (as a source's) of the nearest point of child c of a
+    // node, its ref and end; used = false for an empty slot
+    auto child = [&]( int node, int c, int &ref, int &end ) {
+        float4 const *p = tr.wide + 16 * (int64_t)node + 2 * c;
+        float4 const a = __ldg( p ), b = __ldg( p + 1 );
+        ref = __float_as_int( b.z );
+        end = __float_as_int( b.w );
+        float const gx = fmaxf( 0.f, fmaxf( a.x - tx, tx - a.w ) );
+        float const gy = fmaxf( 0.f, fmaxf( a.y - ty, ty - b.x ) );
+        float const gz = fmaxf( 0.f, fmaxf( a.z - tz, tz - b.y ) );
+        return fmaf( gz, gz, fmaf( gy, gy, gx * gx ) );
+    };
+
+    for ( ;; )
+    {
+        if ( tr.nl == 1 )
+            scan( 0, (int)tr.n );
+        else
+        {
+            int2 stack[NN_LEVELS];
+            int node = 0, sp = 0;
+            unsigned open = 0xffu;
+            bool fresh = true;
+            int64_t steps = 0;
+            for ( ;; )
+            {
+                int next = -1, next_ref = 0, next_end = 0;
+                float next_d = 0.f;
+                unsigned live = 0;
+                auto offer = [&]( int c ) {
+                    int ref, end;
+                    float const d = child( node, c, ref, end );
+                    if ( ref != WIDE_EMPTY && !( d > T ) )
+                    {
+                        live |= 1u << c;
+                        if ( next < 0 || d < next_d )
+                        {
+                            next = c;
+                            next_d = d;
+                            next_ref = ref;
+                            next_end = end;
+                        }
+                    }
+                };
+                if ( fresh )
+                {
+                    // every step enters a wide node, and each at most once
+                    if ( steps++ >= tr.step_cap )
+                    {
+                        atomicOr( status, DEV_TIMEOUT );
+                        break;
+                    }
+#pragma unroll
+                    for ( int c = 0; c < WIDE; ++c )
+                        offer( c );
+                    fresh = false;
+                }
+                else
+                    for ( unsigned m = open; m; m &= m - 1 )
+                        offer( __ffs( m ) - 1 );
+                open = live;
+                if ( next < 0 )
+                {
+                    if ( sp == 0 )
+                        break;
+                    --sp;
+                    node = stack[sp].x;
+                    open = (unsigned)stack[sp].y;
+                    continue;
+                }
+                open &= ~( 1u << next );
+                if ( next_ref >= 0 )
+                {
+                    if ( open )
+                        stack[sp++] = make_int2( node, (int)open );
+                    node = next_ref;
+                    fresh = true;
+                }
+                else
+                    scan( ~next_ref, next_end );
+            }
+        }
+        if ( exact || d_next > T )
+            break;
+        exact = true;
+    }
+    if ( !exact )
+    {
+        ki = (int)__ldg( tr.perm + p_min );
+        kp = p_min;
+    }
+    idx_out[qi] = ki;
+    if ( pos_out )
+        pos_out[qi] = kp;
+}
+
 // Radius traversal shared by the count and fill passes.  FILL=false counts
 // hits into counts[qi]; FILL=true writes them at offset[qi] in traversal
 // order (Morton order of the sources, lane order inside a leaf).  A source
@@ -1921,6 +2103,19 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
     NvtxRange const nvtx_range( "DTK_knn_query" );
     if ( tgt.n == 0 || tree.n == 0 || ( k == 0 && !groups.k ) )
         return;
+    // One query a lane for lists of one, while the warp-per-query kernel would
+    // run three waves of its resident warps or more: with fewer queries it
+    // spreads them over more lanes (2M sources and 20k queries 828 against
+    // 859 us with the tree; 30k and 30k 484 against 454, 2M and 2M 3.97
+    // against 1.86 ms).
+    if ( k == 1 && !groups.tgt_grp && tree.wide_levels <= NN_LEVELS &&
+         tgt.n >= 3 * (int64_t)num_sms() * KNN_BLOCKS_PER_SM * Q_WARPS )
+    {
+        k_nearest<<<blocks_for( tgt.n, NN_THREADS ), NN_THREADS, 0, s>>>( view_of( tree ), tgt, order, idx, pos,
+                                                                          status );
+        check_launch( "k_nearest" );
+        return;
+    }
     GroupView const gv{groups.src_off, groups.tgt_grp, groups.k, groups.r};
     // chunk length: up to Q_SEQ queries, fewer when that leaves under four
     // chunks per resident warp; the last chunk per resident warp is cut in
