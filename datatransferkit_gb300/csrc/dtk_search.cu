@@ -44,6 +44,8 @@
 #include <climits>
 
 #include <algorithm>
+#include <cmath>
+#include <type_traits>
 #include <functional>
 #include <vector>
 
@@ -993,12 +995,13 @@ __device__ __forceinline__ Query make_query( double const *scene, PointsView con
 // round-ups off its issue slots): the search copies the 64-byte record into
 // shared memory with one coalesced load.
 static_assert( sizeof( Query ) == 64, "a query record is 16 words" );
-__global__ void k_query_frame( PointsView tgt, uint32_t const *order, double const *scene, Query *qrec )
+// (n_listed: the length of a list that a kernel wrote, in place of all targets)
+__global__ void k_query_frame( PointsView tgt, uint32_t const *order, double const *scene, Query *qrec,
+                               unsigned const *n_listed = nullptr )
 {
-    int64_t const w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if ( w >= tgt.n )
-        return;
-    qrec[w] = make_query( scene, tgt, order ? (int64_t)order[w] : w );
+    int64_t const n = n_listed ? (int64_t)*n_listed : tgt.n;
+    for ( int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; w < n; w += gridDim.x * (int64_t)blockDim.x )
+        qrec[w] = make_query( scene, tgt, order ? (int64_t)order[w] : w );
 }
 
 // Sorted source p: the FP64 squared distance to the query (the exact key)
@@ -1055,11 +1058,14 @@ constexpr float LIST_GROWTH = 1.5f;
 // seeds the next): n_big chunks of seq queries, then chunks of seq / 2 up to
 // the end, so that the warps finish close together.  A warp takes the next
 // chunk from a counter as soon as it is done with one.
+// Of a list (n_listed, its length on the device) the chunks are as long as
+// leaves four to every warp of the launch, and seq at most.
 struct KnnChunks
 {
     int seq;
     int64_t n_big;
     unsigned *next;
+    unsigned const *n_listed;
 };
 
 __device__ __forceinline__ void chunk_range( KnnChunks const &ch, unsigned c, int64_t &w0, int64_t &len )
@@ -1187,6 +1193,12 @@ __global__ void __launch_bounds__( Q_WARPS * 32, KNN_BLOCKS_PER_SM )
     unsigned const lt_mask = ( 1u << lane ) - 1u;
     if ( lane == 0 )
         s_entry[wib] = 0;
+    int64_t const n_queries = ch.n_listed ? (int64_t)*ch.n_listed : tgt.n;
+    if ( ch.n_listed )
+    {
+        ch.seq = max( 1, min( ch.seq, (int)( n_queries / ( 4 * Q_WARPS * (int64_t)gridDim.x ) ) ) );
+        ch.n_big = n_queries;
+    }
     for ( ;; )
     {
     unsigned c = 0;
@@ -1195,7 +1207,7 @@ __global__ void __launch_bounds__( Q_WARPS * 32, KNN_BLOCKS_PER_SM )
     c = __shfl_sync( FULL, c, 0 );
     int64_t w0, len;
     chunk_range( ch, c, w0, len );
-    if ( w0 >= tgt.n )
+    if ( w0 >= n_queries )
         return;
     if ( lane == 0 )
         s_nlist[wib] = -1;
@@ -1209,7 +1221,7 @@ __global__ void __launch_bounds__( Q_WARPS * 32, KNN_BLOCKS_PER_SM )
     unsigned long long kd = KEY_INF;
     int ki = 0x7fffffff, kp = -1;
     // positions and targets are below 2^31 (int32 offsets): 32-bit loop state
-    int const wb = (int)w0, we = (int)( w0 + len < tgt.n ? w0 + len : tgt.n );
+    int const wb = (int)w0, we = (int)( w0 + len < n_queries ? w0 + len : n_queries );
     bool head = true; // the chunk's first query
     for ( int w = wb; w < we; ++w )
     {
@@ -1611,6 +1623,28 @@ __device__ __forceinline__ float nearest_threshold( float d2, float err )
     return screen_threshold( __fmaf_ru( err, root, rel ), err );
 }
 
+// Squared FP32 distances of a lane's query (centred, tx ty tz): to a source,
+// and to the nearest point of child c of a wide node (with its ref and end).
+__device__ __forceinline__ float lane_dist2( TreeView const &tr, int p, float tx, float ty, float tz )
+{
+    float4 const f = __ldg( tr.f4 + p );
+    float const dx = f.x - tx, dy = f.y - ty, dz = f.z - tz;
+    return fmaf( dz, dz, fmaf( dy, dy, dx * dx ) );
+}
+
+__device__ __forceinline__ float lane_child( TreeView const &tr, int node, int c, float tx, float ty, float tz,
+                                             int &ref, int &end )
+{
+    float4 const *p = tr.wide + 16 * (int64_t)node + 2 * c;
+    float4 const a = __ldg( p ), b = __ldg( p + 1 );
+    ref = __float_as_int( b.z );
+    end = __float_as_int( b.w );
+    float const gx = fmaxf( 0.f, fmaxf( a.x - tx, tx - a.w ) );
+    float const gy = fmaxf( 0.f, fmaxf( a.y - ty, ty - b.x ) );
+    float const gz = fmaxf( 0.f, fmaxf( a.z - tz, tz - b.y ) );
+    return fmaf( gz, gz, fmaf( gy, gy, gx * gx ) );
+}
+
 __global__ void __launch_bounds__( NN_THREADS, NN_BLOCKS_PER_SM )
     k_nearest( TreeView tr, PointsView tgt, uint32_t const *order, int32_t *idx_out, int32_t *pos_out,
                unsigned *status )
@@ -1628,11 +1662,7 @@ __global__ void __launch_bounds__( NN_THREADS, NN_BLOCKS_PER_SM )
     unsigned long long kd = KEY_INF;
     int ki = 0x7fffffff, kp = -1;
 
-    auto dist2 = [&]( int p ) {
-        float4 const f = __ldg( tr.f4 + p );
-        float const dx = f.x - tx, dy = f.y - ty, dz = f.z - tz;
-        return fmaf( dz, dz, fmaf( dy, dy, dx * dx ) );
-    };
+    auto dist2 = [&]( int p ) { return lane_dist2( tr, p, tx, ty, tz ); };
     auto scan = [&]( int start, int end ) {
         if ( exact )
         {
@@ -1667,19 +1697,6 @@ __global__ void __launch_bounds__( NN_THREADS, NN_BLOCKS_PER_SM )
         }
         T = nearest_threshold( d_min, q.err );
     };
-    // squared distance (as a source's) of the nearest point of child c of a
-    // node, its ref and end; used = false for an empty slot
-    auto child = [&]( int node, int c, int &ref, int &end ) {
-        float4 const *p = tr.wide + 16 * (int64_t)node + 2 * c;
-        float4 const a = __ldg( p ), b = __ldg( p + 1 );
-        ref = __float_as_int( b.z );
-        end = __float_as_int( b.w );
-        float const gx = fmaxf( 0.f, fmaxf( a.x - tx, tx - a.w ) );
-        float const gy = fmaxf( 0.f, fmaxf( a.y - ty, ty - b.x ) );
-        float const gz = fmaxf( 0.f, fmaxf( a.z - tz, tz - b.y ) );
-        return fmaf( gz, gz, fmaf( gy, gy, gx * gx ) );
-    };
-
     for ( ;; )
     {
         if ( tr.nl == 1 )
@@ -1698,7 +1715,7 @@ __global__ void __launch_bounds__( NN_THREADS, NN_BLOCKS_PER_SM )
                 unsigned live = 0;
                 auto offer = [&]( int c ) {
                     int ref, end;
-                    float const d = child( node, c, ref, end );
+                    float const d = lane_child( tr, node, c, tx, ty, tz, ref, end );
                     if ( ref != WIDE_EMPTY && !( d > T ) )
                     {
                         live |= 1u << c;
@@ -1761,6 +1778,585 @@ __global__ void __launch_bounds__( NN_THREADS, NN_BLOCKS_PER_SM )
     idx_out[qi] = ki;
     if ( pos_out )
         pos_out[qi] = kp;
+}
+
+// The k nearest sources, 32 queries a warp.
+//
+// A warp a query pays for the tree, the exact FP64 keys and the merges of its
+// list 32 lanes at a time.  Here a warp takes 32 queries that follow each other
+// in Morton order and walks the tree once for all of them, for the leaves in
+// reach of their box.  Then every lane screens the leaves in its own query's
+// reach, at its own pace, and only appends: sources with d2_f <= T go to its
+// column of shared memory, each as one word (20 bits of d2_f / T, then the
+// leaf's place in the list and the source's in the leaf).  T starts a little
+// above the mean k-th distance of the warp's previous 32 queries (of a window
+// of the sources' order for the first); a column that fills up is thinned to a
+// smaller T.  In the end each lane sorts its column in registers (Batcher's
+// merge exchange, 32 words at a time: two instructions a comparator for 32
+// queries at once).  A row is proven when the threshold of its k-th distance is
+// not above T, and searched again with that threshold otherwise.
+//
+// What bounds it is the latency of a warp's own chain, with 16 warps an SM for
+// columns of 72 (45 KB of shared memory a block) and 28 for columns of 40: of a
+// batch of 32 (k = 32, 1M targets) the screens take 49% (13 wavefronts a
+// 128-bit load, the lanes being in different leaves), the sorts 15%, ties 14%,
+// the tree 8%.  Tried and slower at k = 32: columns sorted by the warp, two
+// keys a lane (19% of its issue slots against 15%); every leaf against all
+// lanes from shared memory, two points an instruction (2.6 against 2.3 ms at
+// 1M); a network over all 72 registers (its code left the instruction cache);
+// a walk of the tree by each lane (1.26k instructions a query against 0.9k).
+//
+// The order is the words' wherever neighbours in it are further apart than the
+// FP32 error (the threshold of the k-th less the k-th) and the rounding to 20
+// bits; other rows are put in order with exact FP64 keys.  Queries that do not
+// settle in a few rounds (densities that change by multiples between
+// neighbouring queries, more ties at the k-th than a column holds, squares
+// outside FP32's range) go on a list for k_knn; a warp whose batch failed
+// passes on the batches after it as they are, 1, 3, 7, then 15 between trials,
+// and while a fifth of all batches have failed every warp passes on its chunks.
+// A pilot of 256 batches over all queries runs first, so that a cloud that does
+// not suit is left to k_knn from the start.
+constexpr int KL_THREADS = 128;
+constexpr int KL_WARPS = KL_THREADS / 32;
+constexpr int KL_UNROLL = 8;  // sources a lane screens at a time
+constexpr int KL_CAP_SHORT = 40, KL_BLOCKS_SHORT = 7; // entries of a column, blocks per SM, for rows up to 16
+constexpr int KL_CAP = 72, KL_BLOCKS = 4;             // and for rows up to 32
+constexpr int KL_LIST = 96;   // leaves of a list: three mask words a lane, 7 bits of a word
+constexpr int KL_STACK = 192; // as STACK, for trees of up to NN_LEVELS levels
+constexpr int KL_ROUNDS = 12; // searches of a batch or of parts of it; 4 while most of it is left
+constexpr int KL_THINS = 5;   // of a column in a round
+constexpr int KL_PILOT = 256; // batches of the pilot
+static_assert( LEAF <= 32, "a source's place in its leaf takes 5 bits" );
+
+template <int P, int Q, int R, int D>
+__device__ __forceinline__ void merge_exchange( uint32_t ( &v )[32] )
+{
+#pragma unroll
+    for ( int i = 0; i < 32 - D; ++i )
+        if ( ( i & P ) == R )
+        {
+            uint32_t const a = v[i], b = v[i + D];
+            v[i] = min( a, b );
+            v[i + D] = max( a, b );
+        }
+    if constexpr ( Q != P )
+        merge_exchange<P, Q / 2, P, Q - P>( v );
+    else if constexpr ( P > 1 )
+        merge_exchange<P / 2, 16, 0, P / 2>( v );
+}
+
+__device__ __forceinline__ void sort_32( uint32_t ( &v )[32] )
+{
+    merge_exchange<16, 16, 0, 16>( v );
+}
+
+// v bitonic: ascending
+__device__ __forceinline__ void merge_32( uint32_t ( &v )[32] )
+{
+#pragma unroll
+    for ( int stride = 16; stride > 0; stride >>= 1 )
+#pragma unroll
+        for ( int i = 0; i < 32; ++i )
+            if ( !( i & stride ) )
+            {
+                uint32_t const a = v[i], b = v[i + stride];
+                v[i] = min( a, b );
+                v[i + stride] = max( a, b );
+            }
+}
+
+// The k-th smallest d2_f from query (qx, qy, qz) to the 128 sources around its
+// code in Morton order: a guess of the queries' bound nearby (warp-uniform).
+__device__ __forceinline__ float window_bound( TreeView const &tr, uint32_t code, float qx, float qy, float qz,
+                                               int row, int lane )
+{
+    int64_t const pos = warp_lower_bound( tr.codes, tr.n, code, lane );
+    int64_t s0 = pos - 64;
+    if ( s0 > tr.n - 128 )
+        s0 = tr.n - 128;
+    if ( s0 < 0 )
+        s0 = 0;
+    float d[4];
+#pragma unroll
+    for ( int j = 0; j < 4; ++j )
+    {
+        int64_t const p = s0 + 32 * j + lane;
+        d[j] = p < tr.n ? lane_dist2( tr, (int)p, qx, qy, qz ) : __int_as_float( 0x7f800000 );
+    }
+    // bit by bit from the top: the largest value (to 12 bits of mantissa) with fewer than `row` below it
+    uint32_t v = 0;
+    for ( int bit = 30; bit >= 11; --bit )
+    {
+        float const t = __uint_as_float( v | ( 1u << bit ) );
+        int below = 0;
+#pragma unroll
+        for ( int j = 0; j < 4; ++j )
+            below += __popc( __ballot_sync( FULL, d[j] < t ) );
+        if ( below < row )
+            v |= 1u << bit;
+    }
+    return v < 0x7f800000u ? __uint_as_float( v ) : __int_as_float( 0x7f800000 );
+}
+
+template <int CAP>
+__global__ void __launch_bounds__( KL_THREADS, CAP == KL_CAP_SHORT ? KL_BLOCKS_SHORT : KL_BLOCKS )
+    k_knn_lanes( TreeView tr, PointsView tgt, uint32_t const *order, int row, int per_warp, unsigned *next_chunk,
+                 int64_t pilot_stride, float growth, int32_t const *offset, int32_t *idx_out, int32_t *pos_out,
+                 uint32_t *list,
+                 unsigned *n_listed, unsigned *status )
+{
+    unsigned *const n_failed = n_listed + 1, *const n_settled = n_listed + 2; // batches
+    constexpr int UNROLL = KL_UNROLL;
+    constexpr int FULL_AT = CAP - UNROLL; // a column with more entries takes no more
+    constexpr int PITCH = KL_THREADS + 1; // odd: a column is written down and read across
+    __shared__ uint32_t s_col[CAP][PITCH];
+    __shared__ int s_stack[KL_WARPS][KL_STACK];
+    __shared__ int s_list[KL_WARPS][KL_LIST];   // leaves in reach of the lanes searched (wide node * WIDE + slot)
+    __shared__ int2 s_range[KL_WARPS][KL_LIST]; // and their positions
+    int const lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    unsigned const lt_mask = ( 1u << lane ) - 1u;
+    uint32_t *const cols = &s_col[0][threadIdx.x & ~31], *const col = cols + lane;
+    float const inf = __int_as_float( 0x7f800000 );
+    float spec = inf;
+    int skip = 0, skipped = 0; // batches to pass on, passed on
+    int64_t batch = 0, batch_end = 0;
+    for ( ;; ++batch )
+    {
+        bool const first = batch == batch_end;
+        if ( first )
+        {
+            // the next chunk
+            unsigned c = 0;
+            int pass = 0;
+            if ( pilot_stride )
+            {
+                // one batch a warp, of which only the outcome counts
+                if ( batch_end > 0 )
+                    return;
+                batch = ( blockIdx.x * (int64_t)KL_WARPS + wib ) * pilot_stride;
+                batch_end = batch + 1;
+            }
+            else
+            {
+                if ( lane == 0 )
+                {
+                    c = atomicAdd( next_chunk, 1u );
+                    pass = *(unsigned volatile *)n_failed > *(unsigned volatile *)n_settled / 4u;
+                }
+                batch = (int64_t)__shfl_sync( FULL, c, 0 ) * per_warp;
+                batch_end = batch + per_warp;
+                if ( __shfl_sync( FULL, pass, 0 ) )
+                {
+                    skip = per_warp;
+                    skipped = 0;
+                }
+            }
+        }
+        int64_t const w0 = batch * 32;
+        if ( w0 >= tgt.n )
+            return;
+        // (lanes past the end repeat the last query and write nothing)
+        int const n_real = tgt.n - w0 < 32 ? (int)( tgt.n - w0 ) : 32;
+        int64_t const w = w0 + ( lane < n_real ? lane : n_real - 1 );
+        int const qi = order ? (int)order[w] : (int)w;
+        auto pass_on = [&]( bool mine ) {
+            unsigned const m = __ballot_sync( FULL, mine );
+            unsigned at = 0;
+            if ( lane == 0 && m && !pilot_stride )
+                at = atomicAdd( n_listed, (unsigned)__popc( m ) );
+            at = __shfl_sync( FULL, at, 0 );
+            if ( mine && !pilot_stride )
+                list[at + __popc( m & lt_mask )] = (uint32_t)qi;
+            return __popc( m );
+        };
+        if ( skipped < skip )
+        {
+            // a run of batches, in order
+            int64_t const run = min( (int64_t)( skip - skipped ), batch_end - batch );
+            int64_t const end = min( ( batch + run ) * 32, tgt.n );
+            unsigned at = 0;
+            if ( lane == 0 )
+                at = atomicAdd( n_listed, (unsigned)( end - w0 ) );
+            at = __shfl_sync( FULL, at, 0 );
+            for ( int64_t i = w0 + lane; i < end; i += 32 )
+                list[at + (unsigned)( i - w0 )] = order ? order[i] : (uint32_t)i;
+            skipped += (int)run;
+            batch += run - 1;
+            continue;
+        }
+        int const o = offset[qi];
+        float tx, ty, tz, err;
+        uint32_t code;
+        {
+            Query const q = make_query( tr.scene, tgt, qi );
+            tx = q.tf[0];
+            ty = q.tf[1];
+            tz = q.tf[2];
+            err = q.err;
+            code = morton3( q.tx, q.ty, q.tz, tr.scene );
+        }
+        if ( first || !( spec < inf ) )
+        {
+            // the warp's last chunk was elsewhere: its bound only within
+            // reach of the window's, which is mostly too large
+            int const mid = n_real / 2;
+            float const window = window_bound( tr, __shfl_sync( FULL, code, mid ), __shfl_sync( FULL, tx, mid ),
+                                               __shfl_sync( FULL, ty, mid ), __shfl_sync( FULL, tz, mid ), row, lane );
+            spec = spec > 0.5f * window && spec < window ? spec : window;
+        }
+        float T = spec, kth = inf;
+        bool fin = lane >= n_real, give_up = false;
+        auto exact_key = [&]( int query, int at, unsigned long long &d, int &i ) {
+            double2 const u = __ldg( tr.s2 + 2 * (int64_t)at ), v = __ldg( tr.s2 + 2 * (int64_t)at + 1 );
+            d = (unsigned long long)__double_as_longlong(
+                dist2_rn( u.x, u.y, v.x, tgt( query, 0 ), tgt( query, 1 ), tgt( query, 2 ) ) );
+            i = (int)__double_as_longlong( v.y );
+        };
+        auto position = [&]( uint32_t v ) { return s_range[wib][( v >> 5 ) & 127u].x + (int)( v & 31u ); };
+        unsigned todo = __ballot_sync( FULL, !fin ), sub = 0;
+        for ( int round = 0; todo; ++round )
+        {
+            // the lanes searched together (a split leaves a part of them in sub)
+            sub &= todo;
+            if ( !sub )
+                sub = todo;
+            bool const mine = ( sub >> lane ) & 1u;
+            // d2_f in units of T / 2^20 (less a margin for the rounding)
+            float const scale = 1048500.f / T;
+            bool const enough =
+                round >= ( pilot_stride ? 2 : KL_ROUNDS ) || ( round >= 4 && __popc( todo ) > 16 );
+            if ( mine && ( enough || !( scale > 0.f && scale < 1e38f ) ) )
+                give_up = true; // or T is 0, tiny or infinite
+            if ( __any_sync( FULL, mine && give_up ) )
+            {
+                sub = 0;
+                todo = __ballot_sync( FULL, !fin && !give_up );
+                continue;
+            }
+            // the box of the queries and their largest bound: the FP32
+            // distance to it is at most a lane's own (the same roundings of
+            // smaller gaps)
+            float blo[3] = {mine ? tx : inf, mine ? ty : inf, mine ? tz : inf};
+            float bhi[3] = {mine ? tx : -inf, mine ? ty : -inf, mine ? tz : -inf};
+            float bt = mine ? T : 0.f;
+#pragma unroll
+            for ( int s = 16; s; s >>= 1 )
+            {
+#pragma unroll
+                for ( int d = 0; d < 3; ++d )
+                {
+                    blo[d] = fminf( blo[d], __shfl_xor_sync( FULL, blo[d], s ) );
+                    bhi[d] = fmaxf( bhi[d], __shfl_xor_sync( FULL, bhi[d], s ) );
+                }
+                bt = fmaxf( bt, __shfl_xor_sync( FULL, bt, s ) );
+            }
+            int n = 0, p = 0, e = 0, base = 0, sp = 0, n_list = 0, thins = 0;
+            uint32_t ref = 0; // the word's low bits of position p
+            unsigned m0 = 0, m1 = 0, m2 = 0;
+            bool walking = tr.nl > 1, again = false;
+            int const grp = lane >> 3, slot = lane & 7;
+            int node = grp == 0 ? 0 : -1;
+            int64_t steps = 0;
+            // the leaves in reach
+            if ( tr.nl == 1 )
+            {
+                if ( lane == 0 )
+                    s_range[wib][0] = make_int2( 0, (int)tr.n );
+                __syncwarp();
+            }
+            while ( walking )
+            {
+                // every step enters at least one wide node, and each is entered at most once
+                if ( steps++ >= tr.step_cap )
+                {
+                    if ( lane == 0 )
+                        atomicOr( status, DEV_TIMEOUT );
+                    give_up = give_up || mine;
+                    n_list = 0;
+                    break;
+                }
+                bool cand = false;
+                int child = WIDE_EMPTY, lend = 0;
+                if ( node >= 0 )
+                {
+                    float lo[3], hi[3], g[3];
+                    int rlo = 0, rhi = 0;
+                    load_wide<false>( tr.wide, nullptr, node, slot, lo, hi, child, lend, rlo, rhi );
+#pragma unroll
+                    for ( int d = 0; d < 3; ++d )
+                        g[d] = fmaxf( 0.f, fmaxf( lo[d] - bhi[d], blo[d] - hi[d] ) );
+                    cand = child != WIDE_EMPTY && !( fmaf( g[2], g[2], fmaf( g[1], g[1], g[0] * g[0] ) ) > bt );
+                }
+                unsigned const ml = __ballot_sync( FULL, cand && child < 0 );
+                unsigned const mi = __ballot_sync( FULL, cand && child >= 0 );
+                int const n_int = __popc( mi ), n_leaf = __popc( ml );
+                if ( n_list + n_leaf > KL_LIST )
+                {
+                    again = true;
+                    break;
+                }
+                if ( sp + n_int <= KL_STACK )
+                {
+                    if ( cand && child >= 0 )
+                        s_stack[wib][sp + __popc( mi & lt_mask )] = child;
+                    sp += n_int;
+                }
+                else if ( lane == 0 )
+                    atomicOr( status, DEV_STACK_OVERFLOW );
+                if ( cand && child < 0 )
+                {
+                    int const at = n_list + __popc( ml & lt_mask );
+                    s_list[wib][at] = node * WIDE + slot;
+                    s_range[wib][at] = make_int2( ~child, lend );
+                }
+                n_list += n_leaf;
+                __syncwarp();
+                // as the query traversal: four nodes a step while a descent fits
+                int const P = sp + ( NODE_GROUPS + tr.levels ) * ( WIDE - 1 ) <= KL_STACK ? NODE_GROUPS : 1;
+                int const taken = sp < P ? sp : P;
+                walking = taken > 0;
+                node = grp < taken ? s_stack[wib][sp - 1 - grp] : -1;
+                sp -= taken;
+                __syncwarp();
+            }
+            if ( again )
+            {
+                // too many leaves: the queries of the lower cell alone
+                uint32_t const c0 = __shfl_sync( FULL, code, __ffs( sub ) - 1 );
+                uint32_t const diff = __reduce_or_sync( FULL, mine ? code ^ c0 : 0u );
+                if ( diff )
+                    sub = __ballot_sync( FULL, mine && !( ( ( code ^ c0 ) >> ( 31 - __clz( diff ) ) ) & 1u ) );
+                else
+                    give_up = give_up || mine;
+                todo = __ballot_sync( FULL, !fin && !give_up );
+                continue;
+            }
+            // each lane's own leaves of the list
+            base = 0;
+#pragma unroll
+            for ( int word = 0; word < 3; ++word )
+            {
+                unsigned m = 0;
+                int const cnt = min( 32, n_list - 32 * word );
+#pragma unroll 4
+                for ( int i = 0; i < cnt; ++i )
+                {
+                    unsigned const at = (unsigned)s_list[wib][32 * word + i];
+                    int cref, cend;
+                    if ( !( lane_child( tr, at / WIDE, at % WIDE, tx, ty, tz, cref, cend ) > T ) )
+                        m |= 1u << i;
+                }
+                if ( tr.nl == 1 )
+                    m = word == 0;
+                ( word == 0 ? m0 : word == 1 ? m1 : m2 ) = mine && !give_up ? m : 0u;
+            }
+            // screen them, each lane at its own pace
+            while ( __any_sync( FULL, p < e || ( m0 | m1 | m2 ) ) )
+            {
+                if ( p >= e )
+                {
+                    if ( !m0 )
+                    {
+                        m0 = m1;
+                        m1 = m2;
+                        m2 = 0;
+                        base += 32;
+                    }
+                    if ( m0 )
+                    {
+                        int const at = base + __ffs( m0 ) - 1;
+                        int2 const r = s_range[wib][at];
+                        m0 &= m0 - 1;
+                        p = r.x;
+                        e = r.y;
+                        ref = (uint32_t)at << 5;
+                    }
+                }
+                if ( p < e )
+                {
+                    float d[UNROLL];
+#pragma unroll
+                    for ( int j = 0; j < UNROLL; ++j )
+                        d[j] = lane_dist2( tr, min( p + j, e - 1 ), tx, ty, tz );
+#pragma unroll
+                    for ( int j = 0; j < UNROLL; ++j )
+                    {
+                        // (2^23 + q as a float has q in its low bits)
+                        col[n * PITCH] =
+                            __float_as_uint( fmaf( d[j], scale, 8388608.f ) ) * 4096u + ( ref + (uint32_t)j );
+                        n += p + j < e && d[j] <= T ? 1 : 0;
+                    }
+                    p += UNROLL;
+                    ref += UNROLL;
+                    while ( n > FULL_AT )
+                    {
+                        // thin the column to 0.85 T (about 0.78 of it),
+                        // faster when that was too little
+                        if ( ++thins > KL_THINS )
+                        {
+                            give_up = true;
+                            n = p = e = 0;
+                            m0 = m1 = m2 = 0;
+                            break;
+                        }
+                        T *= thins < 3 ? 0.85f : 0.5f;
+                        uint32_t const cut = ( (uint32_t)( T * scale ) + 2u ) << 12;
+                        int m = 0;
+                        for ( int i = 0; i < n; ++i )
+                        {
+                            uint32_t const v = col[i * PITCH];
+                            col[m * PITCH] = v;
+                            m += v < cut ? 1 : 0;
+                        }
+                        n = m;
+                    }
+                }
+            }
+            __syncwarp();
+            sub = 0;
+            bool out = false, tie = false;
+            uint32_t cut = 0;
+            if ( mine && !give_up && n >= row )
+            {
+                // the 32 smallest words in order, in the column's first 32
+                // entries, the others behind them in any order
+                int const blocks = ( n + 31 ) / 32;
+                uint32_t v[32];
+                for ( int k = blocks - 1; k >= 0; --k )
+                {
+#pragma unroll
+                    for ( int i = 0; i < 32; ++i )
+                        v[i] = 32 * k + i < n ? col[( 32 * k + i ) * PITCH] : 0xffffffffu;
+                    sort_32( v );
+                    if ( k > 0 )
+                    {
+#pragma unroll
+                        for ( int i = 0; i < 32; ++i )
+                            if ( 32 * k + i < n )
+                                col[( 32 * k + i ) * PITCH] = v[i];
+                    }
+                }
+                uint32_t rest = 0xffffffffu; // the smallest word behind them
+                for ( int k = 1; k < blocks; ++k )
+                {
+#pragma unroll
+                    for ( int i = 0; i < 32; ++i )
+                        if ( 32 * k + 31 - i < n )
+                        {
+                            uint32_t const u = col[( 32 * k + 31 - i ) * PITCH];
+                            uint32_t const behind = max( v[i], u );
+                            col[( 32 * k + 31 - i ) * PITCH] = behind;
+                            rest = min( rest, behind );
+                            v[i] = min( v[i], u );
+                        }
+                    merge_32( v );
+                }
+                uint32_t kk = 0;
+#pragma unroll
+                for ( int i = 0; i < 32; ++i )
+                    kk = i == row - 1 ? v[i] : kk;
+                kk >>= 12;
+                // (a word's d2_f lies within one unit of it)
+                float const unit = __fdiv_ru( 1.f, scale ) * 1.000001f;
+                float const hi = __fmul_ru( (float)( kk + 1u ), unit );
+                float const bound = nearest_threshold( hi, err );
+                uint32_t const cut_q = (uint32_t)fminf( bound * scale, 1048570.f ) + 2u;
+                cut = cut_q << 12;
+                // words of the row closer than the error are not in order yet,
+                // nor is its last when others are within the error of it
+                uint32_t const tol = ( min( cut_q - kk + 3u, 0xfffffu ) << 12 ) | 4095u;
+#pragma unroll
+                for ( int i = 0; i < 31; ++i )
+                    tie |= i < row - 1 && v[i + 1] - v[i] <= tol;
+#pragma unroll
+                for ( int i = 0; i < 32; ++i )
+                    tie |= i >= row && v[i] < cut;
+                tie |= rest < cut;
+#pragma unroll
+                for ( int i = 0; i < 32; ++i )
+                    if ( i < n )
+                        col[i * PITCH] = v[i];
+                if ( bound <= T )
+                {
+                    out = true;
+                    fin = true;
+                    kth = hi;
+                }
+                else
+                    T = bound; // not proven: once more
+            }
+            else if ( mine )
+                T *= 1.6f; // too few
+            __syncwarp();
+            unsigned const rows = __ballot_sync( FULL, out && !tie );
+#pragma unroll 4
+            for ( int j = 0; j < 32; ++j )
+            {
+                int const at = __shfl_sync( FULL, o, j ) + lane;
+                if ( ( ( rows >> j ) & 1u ) && lane < row )
+                {
+                    int const pos = position( cols[lane * PITCH + j] );
+                    idx_out[at] = (int32_t)__ldg( tr.perm + pos );
+                    if ( pos_out )
+                        pos_out[at] = pos;
+                }
+            }
+            for ( unsigned ties = __ballot_sync( FULL, out && tie ); ties; ties &= ties - 1 )
+            {
+                // every word that may belong to the row, by exact key
+                int const j = __ffs( ties ) - 1;
+                int const nj = __shfl_sync( FULL, n, j ), qj = __shfl_sync( FULL, qi, j );
+                uint32_t const cut_j = __shfl_sync( FULL, cut, j );
+                unsigned long long d = KEY_INF;
+                int i = 0x7fffffff, pos = 0;
+                for ( int k = 0; k < nj; k += 32 )
+                {
+                    uint32_t const v = k + lane < nj ? cols[( k + lane ) * PITCH + j] : 0xffffffffu;
+                    if ( !__any_sync( FULL, v < cut_j ) )
+                        continue;
+                    unsigned long long d2 = KEY_INF;
+                    int i2 = 0x7fffffff, pos2 = 0;
+                    if ( v < cut_j )
+                    {
+                        pos2 = position( v );
+                        exact_key( qj, pos2, d2, i2 );
+                    }
+                    sort_entries<true>( d2, i2, pos2, lane );
+                    // into the list, as the reversed sequence
+                    d2 = __shfl_sync( FULL, d2, 31 - lane );
+                    i2 = __shfl_sync( FULL, i2, 31 - lane );
+                    pos2 = __shfl_sync( FULL, pos2, 31 - lane );
+                    if ( key_less( d2, i2, d, i ) )
+                    {
+                        d = d2;
+                        i = i2;
+                        pos = pos2;
+                    }
+                    sort_entries<false>( d, i, pos, lane );
+                }
+                int const at = __shfl_sync( FULL, o, j ) + lane;
+                if ( lane < row )
+                {
+                    idx_out[at] = i;
+                    if ( pos_out )
+                        pos_out[at] = pos;
+                }
+            }
+            __syncwarp();
+            todo = __ballot_sync( FULL, !fin && !give_up );
+        }
+        bool const failed = pass_on( give_up ) > n_real / 2;
+        skip = failed ? min( 2 * skip + 1, 15 ) : 0;
+        skipped = 0;
+        if ( lane == 0 )
+            atomicAdd( failed ? n_failed : n_settled, 1u );
+        float sum = kth < inf ? kth : 0.f;
+        int const got = __popc( __ballot_sync( FULL, kth < inf ) );
+#pragma unroll
+        for ( int s = 16; s; s >>= 1 )
+            sum += __shfl_xor_sync( FULL, sum, s );
+        spec = got ? sum / got * growth : inf;
+    }
 }
 
 // Radius traversal shared by the count and fill passes.  FILL=false counts
@@ -2130,10 +2726,49 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
     int64_t const n_chunks = n_big + ( tgt.n - n_big * seq + tail - 1 ) / tail;
     int64_t const warps = n_chunks < resident ? n_chunks : resident;
     unsigned const blocks = blocks_for( warps, Q_WARPS );
-    DeviceBuffer<unsigned> next( 1, s );
-    DTK_CUDA_OR_THROW( cudaMemsetAsync( next.get(), 0, sizeof( unsigned ), s ) );
-    KnnChunks const ch{seq, n_big, next.get()};
+    // chunk counters of k_knn and of k_knn_lanes; the list's length, failed and settled batches
+    DeviceBuffer<unsigned> next( 5, s );
+    DTK_CUDA_OR_THROW( cudaMemsetAsync( next.get(), 0, 5 * sizeof( unsigned ), s ) );
     DeviceBuffer<Query> qrec( tgt.n, s );
+    // 32 queries a warp, in columns of 40 for rows up to 16 and of 72 above,
+    // from 6 and 24 batches a resident warp on: below that the pilot and the
+    // warps' first batches, whose bounds are rough, take what the others save.
+    // Search with the tree, k_knn alone against this: k = 8, 800k targets 1.97
+    // / 1.73 ms, 2M 4.28 / 3.10, 8M 15.2 / 9.6; k = 20, 2M 4.39 / 4.00 (1M 2.46
+    // / 2.31), 8M 15.6 / 13.1; k = 32, 1M 2.77 / 2.93, 2M 5.01 / 4.89, 8M 17.5
+    // / 16.1.  At 3M and k = 20: grid 7.5 / 6.9, sphere 5.5 / 5.1, clusters 6.8
+    // / 7.1, duplicates 10.1 / 9.5, targets far outside 5.6 / 5.6.
+    int const row = (int)std::min<int64_t>( k, tree.n );
+    int const lane_blocks = num_sms() * ( row <= 16 ? KL_BLOCKS_SHORT : KL_BLOCKS );
+    int64_t const lane_warps = (int64_t)lane_blocks * KL_WARPS;
+    if ( !groups.tgt_grp && tree.wide_levels <= NN_LEVELS && tgt.n >= ( row <= 16 ? 192 : 768 ) * lane_warps )
+    {
+        int const cap = row <= 16 ? KL_CAP_SHORT : KL_CAP;
+        // the bound from the mean k-th distance: so that it holds 1.6 to 2
+        // times the row, 0.7 of the column at most (1.2 rows and the searches
+        // again cost more than the points saved, 2.2 and the columns overflow)
+        float const growth = (float)std::pow( std::min( 2.0, 0.7 * cap / row ), 2.0 / 3.0 );
+        int const per_warp = (int)std::min<int64_t>( 16, std::max<int64_t>( 1, tgt.n / 32 / ( 4 * lane_warps ) ) );
+        DeviceBuffer<uint32_t> list( tgt.n, s );
+        auto const kernel = row <= 16 ? k_knn_lanes<KL_CAP_SHORT> : k_knn_lanes<KL_CAP>;
+        int64_t const batches = ( tgt.n + 31 ) / 32;
+        kernel<<<KL_PILOT / KL_WARPS, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, 1, next.get() + 1,
+                                                           batches / KL_PILOT, growth, offset, idx, pos, list.get(),
+                                                           next.get() + 2, status );
+        check_launch( "k_knn_lanes(pilot)" );
+        kernel<<<lane_blocks, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, per_warp, next.get() + 1, 0,
+                                                   growth, offset, idx, pos, list.get(), next.get() + 2, status );
+        check_launch( "k_knn_lanes" );
+        // what it left
+        k_query_frame<<<8 * num_sms(), 256, 0, s>>>( tgt, list.get(), tree.scene.get(), qrec.get(), next.get() + 2 );
+        check_launch( "k_query_frame" );
+        KnnChunks const rest{Q_SEQ, 0, next.get(), next.get() + 2};
+        k_knn<false><<<num_sms() * KNN_BLOCKS_PER_SM, Q_WARPS * 32, 0, s>>>(
+            view_of( tree ), tgt, list.get(), qrec.get(), k, rest, gv, offset, idx, pos, status );
+        check_launch( "k_knn" );
+        return;
+    }
+    KnnChunks const ch{seq, n_big, next.get(), nullptr};
     k_query_frame<<<blocks_for( tgt.n, 256 ), 256, 0, s>>>( tgt, order, tree.scene.get(), qrec.get() );
     check_launch( "k_query_frame" );
     if ( groups.tgt_grp )
