@@ -8,16 +8,17 @@
 // into one kernel that reads idx/coeff once and writes each target once.
 //
 // Rows of equal length R with R % 4 == 0 and R/4 a power of two (kNN rows,
-// e.g. R = 32) use R/8 lanes per row (8 entries each; R/4 lanes of 4 for
-// FP64 coefficients) with 128-bit loads:
+// e.g. R = 32) use R/8 lanes per row (8 entries each) with 128-bit loads:
 // int4 of indices and two double2 (FP64 form) or one float4 (mixed form) of
-// coefficients per 4 entries, then a shuffle reduction.  Other rows use S lanes per row (S a power of two chosen
-// from the mean row length) with coalesced scalar loads.  Source values are
+// coefficients per 4 entries, then a shuffle reduction.  Other rows use S lanes
+// per row (S a power of two chosen from the mean row length) with coalesced
+// scalar loads.  Source values are
 // gathered through the read-only path; at 8M sources they are 64 MB and stay
 // resident in the 129 MB L2 while the CSR streams from HBM.
 #include "dtk_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace dtk
 {
@@ -33,47 +34,6 @@ __device__ __forceinline__ double group_sum( double v )
     for ( int o = L / 2; o > 0; o >>= 1 )
         v += __shfl_xor_sync( FULL, v, o );
     return v;
-}
-
-// L lanes per row, each lane EPL consecutive entries (EPL a multiple of 4).
-template <int L, int EPL, bool F32>
-__global__ void __launch_bounds__( 256 )
-    k_apply_vec( int64_t n_tgt, int32_t const *__restrict__ idx,
-                 void const *__restrict__ coeff, double const *__restrict__ values,
-                 double *__restrict__ target )
-{
-    constexpr int R = EPL * L;
-    int64_t const gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    int64_t const row = gt / L;
-    int const sub = (int)( gt % L );
-    double acc = 0.0;
-    if ( row < n_tgt )
-    {
-#pragma unroll
-        for ( int q = 0; q < EPL; q += 4 )
-        {
-            int64_t const e = row * R + EPL * sub + q;
-            int4 const ix = __ldcs( reinterpret_cast<int4 const *>( idx + e ) );
-            if constexpr ( F32 )
-            {
-                float4 const c =
-                    __ldcs( reinterpret_cast<float4 const *>( static_cast<float const *>( coeff ) + e ) );
-                acc += (double)c.x * __ldg( values + ix.x ) + (double)c.y * __ldg( values + ix.y ) +
-                       (double)c.z * __ldg( values + ix.z ) + (double)c.w * __ldg( values + ix.w );
-            }
-            else
-            {
-                double const *cp = static_cast<double const *>( coeff ) + e;
-                double2 const c0 = __ldcs( reinterpret_cast<double2 const *>( cp ) );
-                double2 const c1 = __ldcs( reinterpret_cast<double2 const *>( cp + 2 ) );
-                acc += c0.x * __ldg( values + ix.x ) + c0.y * __ldg( values + ix.y ) +
-                       c1.x * __ldg( values + ix.z ) + c1.y * __ldg( values + ix.w );
-            }
-        }
-    }
-    acc = group_sum<L>( acc );
-    if ( row < n_tgt && sub == 0 )
-        target[row] = acc;
 }
 
 // S lanes per row, strided scalar loads.
@@ -100,46 +60,6 @@ __global__ void __launch_bounds__( 256 )
     acc = group_sum<S>( acc );
     if ( row < n_tgt && sub == 0 )
         target[row] = acc;
-}
-
-// Row length R = 4 * 2^j (at most 128): R / EPL lanes per row, each EPL
-// entries (4 entries a lane for rows shorter than EPL).  FP32 coefficients
-// take EPL = 8 (one reduction level fewer: -9% at 8M x 32), FP64 ones 4
-// (twice the coefficient bytes a lane: +5% at 8).
-template <bool F32>
-constexpr int apply_epl()
-{
-    return F32 ? 8 : 4;
-}
-
-template <int EPL, bool F32>
-void launch_vec_epl( int L, unsigned blocks, int64_t n_tgt, int32_t const *idx, void const *coeff,
-                     double const *values, double *target, cudaStream_t s )
-{
-    switch ( L )
-    {
-    case 1: k_apply_vec<1, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, idx, coeff, values, target ); break;
-    case 2: k_apply_vec<2, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, idx, coeff, values, target ); break;
-    case 4: k_apply_vec<4, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, idx, coeff, values, target ); break;
-    case 8: k_apply_vec<8, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, idx, coeff, values, target ); break;
-    case 16: k_apply_vec<16, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, idx, coeff, values, target ); break;
-    default: k_apply_vec<32, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, idx, coeff, values, target ); break;
-    }
-}
-
-template <bool F32>
-void launch_vec( int R, int64_t n_tgt, int32_t const *idx, void const *coeff,
-                 double const *values, double *target, cudaStream_t s )
-{
-    constexpr int EPL = apply_epl<F32>();
-    int const epl = R >= EPL ? EPL : 4;
-    int const L = R / epl;
-    unsigned const blocks = (unsigned)( ( n_tgt * L + 255 ) / 256 );
-    if ( epl == EPL )
-        launch_vec_epl<EPL, F32>( L, blocks, n_tgt, idx, coeff, values, target, s );
-    else
-        launch_vec_epl<4, F32>( L, blocks, n_tgt, idx, coeff, values, target, s );
-    check_launch( "k_apply_vec" );
 }
 
 template <bool F32>
@@ -173,7 +93,14 @@ bool is_pow2( int v ) { return v > 0 && ( v & ( v - 1 ) ) == 0; }
 // fl32(v - hi)) and sums c_j (hi_j + lo_j) in double-float arithmetic on the
 // FP32 pipe (TwoProd / TwoSum, the compensated scheme of the mixed setup):
 // the FP32 coefficients are the only rounding left, as with an FP64 sum.
-// The FP64 form permutes the doubles and sums with FP64 FMAs.  Rows go in
+// The FP64 form permutes the doubles and sums with FP64 FMAs, whose pipe bounds
+// it (64 cycles an instruction a warp): one FMA an entry, and the lanes' partial
+// sums of a row are added for as many rows as there are lanes at once, each
+// lane ending with one row (2M rows of 32 with the permutation 257 -> 201 us,
+// 118 us of them the bytes).  A field of several
+// components keeps a point's components side by side, up to four a pass, so
+// that positions and coefficients are read once (three components of 1M rows of
+// 32, mixed: 480 -> 143 us against FP64 sums by index).  Rows go in
 // the targets' Morton order when the operator has it, so that consecutive
 // rows share most of their neighbours' values in L1 (0.70 -> 0.59 ms for 8M
 // rows of 32; 16 entries a lane instead of 8 was 1.26 ms, 4 no different).
@@ -223,84 +150,175 @@ __device__ __forceinline__ void df_axpy( float c, float2 v, float &s, float &cs 
     cs = __fadd_rn( cs, __fadd_rn( f, e ) );
 }
 
-// L lanes per row, each lane EPL consecutive entries (EPL a multiple of 4).
-template <int L, int EPL, bool F32>
+// The double-floats (s, cs) of a group of L lanes added up.
+template <int L>
+__device__ __forceinline__ double df_group_sum( float s, float cs )
+{
+#pragma unroll
+    for ( int o = L / 2; o > 0; o >>= 1 )
+    {
+        float const os = __shfl_xor_sync( FULL, s, o ), oc = __shfl_xor_sync( FULL, cs, o );
+        float t, f;
+        two_sum( s, os, t, f );
+        s = t;
+        cs = __fadd_rn( cs, __fadd_rn( oc, f ) );
+    }
+    return (double)s + (double)cs;
+}
+
+// Mixed form: L lanes per row, each lane EPL consecutive entries (EPL a
+// multiple of 4), CB components.
+template <int L, int EPL, int CB>
 __global__ void __launch_bounds__( 256 )
-    k_apply_pos( int64_t n_tgt, int32_t const *__restrict__ pos, void const *__restrict__ coeff,
-                 void const *__restrict__ sorted, double *__restrict__ target, uint32_t const *__restrict__ order )
+    k_apply_pos( int64_t n_tgt, int32_t const *__restrict__ pos, float const *__restrict__ coeff,
+                 float2 const *__restrict__ sorted, double *__restrict__ target, int64_t ps, int64_t cs_out,
+                 uint32_t const *__restrict__ order )
 {
     constexpr int R = EPL * L;
     int64_t const gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t const row0 = gt / L;
     int64_t const row = ( order && row0 < n_tgt ) ? (int64_t)__ldg( order + row0 ) : row0;
     int const sub = (int)( gt % L );
-    if constexpr ( F32 )
+    float s[CB] = {}, cs[CB] = {};
+    if ( row < n_tgt )
     {
-        float2 const *vals = static_cast<float2 const *>( sorted );
-        float s = 0.f, cs = 0.f;
-        if ( row < n_tgt )
-        {
 #pragma unroll
-            for ( int q = 0; q < EPL; q += 4 )
+        for ( int q = 0; q < EPL; q += 4 )
+        {
+            int64_t const e = row * R + EPL * sub + q;
+            int4 const ix = __ldcs( reinterpret_cast<int4 const *>( pos + e ) );
+            float4 const c = __ldcs( reinterpret_cast<float4 const *>( coeff + e ) );
+            int const at[4] = {ix.x, ix.y, ix.z, ix.w};
+            float const cj[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+            for ( int j = 0; j < 4; ++j )
             {
-                int64_t const e = row * R + EPL * sub + q;
-                int4 const ix = __ldcs( reinterpret_cast<int4 const *>( pos + e ) );
-                float4 const c =
-                    __ldcs( reinterpret_cast<float4 const *>( static_cast<float const *>( coeff ) + e ) );
-                df_axpy( c.x, __ldg( vals + ix.x ), s, cs );
-                df_axpy( c.y, __ldg( vals + ix.y ), s, cs );
-                df_axpy( c.z, __ldg( vals + ix.z ), s, cs );
-                df_axpy( c.w, __ldg( vals + ix.w ), s, cs );
+                float2 const *v = sorted + (int64_t)CB * at[j];
+#pragma unroll
+                for ( int k = 0; k < CB; ++k )
+                    df_axpy( cj[j], __ldg( v + k ), s[k], cs[k] );
             }
         }
-#pragma unroll
-        for ( int o = L / 2; o > 0; o >>= 1 )
-        {
-            float const os = __shfl_xor_sync( FULL, s, o ), oc = __shfl_xor_sync( FULL, cs, o );
-            float t, f;
-            two_sum( s, os, t, f );
-            s = t;
-            cs = __fadd_rn( cs, __fadd_rn( oc, f ) );
-        }
-        if ( row < n_tgt && sub == 0 )
-            target[row] = (double)s + (double)cs;
     }
-    else
-    {
-        double const *vals = static_cast<double const *>( sorted );
-        double acc = 0.0;
-        if ( row < n_tgt )
-        {
 #pragma unroll
-            for ( int q = 0; q < EPL; q += 4 )
-            {
-                int64_t const e = row * R + EPL * sub + q;
-                int4 const ix = __ldcs( reinterpret_cast<int4 const *>( pos + e ) );
-                double const *cp = static_cast<double const *>( coeff ) + e;
-                double2 const c0 = __ldcs( reinterpret_cast<double2 const *>( cp ) );
-                double2 const c1 = __ldcs( reinterpret_cast<double2 const *>( cp + 2 ) );
-                acc += c0.x * __ldg( vals + ix.x ) + c0.y * __ldg( vals + ix.y ) +
-                       c1.x * __ldg( vals + ix.z ) + c1.y * __ldg( vals + ix.w );
-            }
-        }
-        acc = group_sum<L>( acc );
+    for ( int k = 0; k < CB; ++k )
+    {
+        double const sum = df_group_sum<L>( s[k], cs[k] );
         if ( row < n_tgt && sub == 0 )
-            target[row] = acc;
+            target[row * ps + k * cs_out] = sum;
     }
 }
 
-template <int EPL, bool F32>
-void launch_pos_epl( int L, unsigned blocks, int64_t n_tgt, int32_t const *pos, void const *coeff,
-                     void const *sorted, double *target, cudaStream_t s, uint32_t const *order )
+// FP64 form: L lanes take L rows, each lane EPL consecutive entries of every
+// row (EPL a multiple of 4), CB components; lane sub ends with row sub.
+template <int L, int EPL, int CB>
+__global__ void __launch_bounds__( 256 )
+    k_apply_pos64( int64_t n_tgt, int32_t const *__restrict__ pos, double const *__restrict__ coeff,
+                   double const *__restrict__ sorted, double *__restrict__ target, int64_t ps, int64_t cs_out,
+                   uint32_t const *__restrict__ order )
 {
-    switch ( L )
+    constexpr int R = EPL * L;
+    int64_t const at0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; // this lane's row in order
+    int const sub = threadIdx.x % L;
+    int64_t const mine = at0 < n_tgt ? ( order ? (int64_t)__ldg( order + at0 ) : at0 ) : -1;
+    double a[L][CB];
+#pragma unroll
+    for ( int r = 0; r < L; ++r )
     {
-    case 1: k_apply_pos<1, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, pos, coeff, sorted, target, order ); break;
-    case 2: k_apply_pos<2, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, pos, coeff, sorted, target, order ); break;
-    case 4: k_apply_pos<4, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, pos, coeff, sorted, target, order ); break;
-    case 8: k_apply_pos<8, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, pos, coeff, sorted, target, order ); break;
-    case 16: k_apply_pos<16, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, pos, coeff, sorted, target, order ); break;
-    default: k_apply_pos<32, EPL, F32><<<blocks, 256, 0, s>>>( n_tgt, pos, coeff, sorted, target, order ); break;
+#pragma unroll
+        for ( int k = 0; k < CB; ++k )
+            a[r][k] = 0.0;
+        int64_t const row = L > 1 ? __shfl_sync( FULL, mine, r, L ) : mine;
+        if ( row < 0 )
+            continue;
+#pragma unroll
+        for ( int q = 0; q < EPL; q += 4 )
+        {
+            int64_t const e = row * R + EPL * sub + q;
+            int4 const ix = __ldcs( reinterpret_cast<int4 const *>( pos + e ) );
+            double2 const c0 = __ldcs( reinterpret_cast<double2 const *>( coeff + e ) );
+            double2 const c1 = __ldcs( reinterpret_cast<double2 const *>( coeff + e + 2 ) );
+            int const at[4] = {ix.x, ix.y, ix.z, ix.w};
+            double const cj[4] = {c0.x, c0.y, c1.x, c1.y};
+#pragma unroll
+            for ( int j = 0; j < 4; ++j )
+            {
+                double const *v = sorted + (int64_t)CB * at[j];
+#pragma unroll
+                for ( int k = 0; k < CB; ++k )
+                    a[r][k] = fma( cj[j], __ldg( v + k ), a[r][k] );
+            }
+        }
+    }
+    // halve the rows a lane holds until one is left
+#pragma unroll
+    for ( int o = L / 2; o > 0; o >>= 1 )
+    {
+        bool const upper = ( sub & o ) != 0;
+#pragma unroll
+        for ( int r = 0; r < o; ++r )
+#pragma unroll
+            for ( int k = 0; k < CB; ++k )
+            {
+                double const give = upper ? a[r][k] : a[r + o][k];
+                double const keep = upper ? a[r + o][k] : a[r][k];
+                a[r][k] = keep + __shfl_xor_sync( FULL, give, o );
+            }
+    }
+    if ( mine >= 0 )
+#pragma unroll
+        for ( int k = 0; k < CB; ++k )
+            target[mine * ps + k * cs_out] = a[0][k];
+}
+
+// sorted[CB p + k] = component c0 + k of source perm[p]
+template <int CB>
+__global__ void k_permute_fields( FieldView in, int64_t c0, uint32_t const *__restrict__ perm,
+                                  double *__restrict__ sorted64, float2 *__restrict__ sorted32 )
+{
+    int64_t const p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if ( p >= in.n )
+        return;
+    double const *v = in.base + ( perm ? (int64_t)__ldg( perm + p ) : p ) * in.ps + c0 * in.cs;
+#pragma unroll
+    for ( int k = 0; k < CB; ++k )
+    {
+        double const x = __ldg( v + k * in.cs );
+        if ( sorted32 )
+        {
+            float const hi = __double2float_rn( x );
+            sorted32[CB * p + k] = make_float2( hi, __double2float_rn( x - (double)hi ) );
+        }
+        else
+            sorted64[CB * p + k] = x;
+    }
+}
+
+// CB components of the rows; v64, v32: the values that pos points into.
+template <int CB>
+void launch_pos( int64_t n_rows, int R, int32_t const *pos, double const *coeff64, float const *coeff32,
+                 double const *v64, float2 const *v32, double *target, int64_t ps, int64_t cs, cudaStream_t s,
+                 uint32_t const *order )
+{
+    auto const run = [&]( auto l, auto epl ) {
+        constexpr int L = decltype( l )::value, EPL = decltype( epl )::value;
+        if ( coeff32 )
+            k_apply_pos<L, EPL, CB><<<(unsigned)( ( n_rows * L + 255 ) / 256 ), 256, 0, s>>>(
+                n_rows, pos, coeff32, v32, target, ps, cs, order );
+        else
+            k_apply_pos64<L, EPL, CB><<<(unsigned)( ( n_rows + 255 ) / 256 ), 256, 0, s>>>(
+                n_rows, pos, coeff64, v64, target, ps, cs, order );
+        check_launch( "k_apply_pos" );
+    };
+    std::integral_constant<int, 8> const eight;
+    switch ( R )
+    {
+    case 4: run( std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{} ); break;
+    case 8: run( std::integral_constant<int, 1>{}, eight ); break;
+    case 16: run( std::integral_constant<int, 2>{}, eight ); break;
+    case 32: run( std::integral_constant<int, 4>{}, eight ); break;
+    case 64: run( std::integral_constant<int, 8>{}, eight ); break;
+    default: run( std::integral_constant<int, 16>{}, eight ); break;
     }
 }
 
@@ -331,26 +349,9 @@ SortedValues permute_values( int64_t n_src, uint32_t const *perm, double const *
 void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double const *coeff64, float const *coeff32,
                 SortedValues const &v, double *target, cudaStream_t s, uint32_t const *order )
 {
-    if ( n_rows == 0 )
-        return;
-    int const R = uniform_row;
-    if ( coeff32 )
-    {
-        int const epl = R >= 8 ? 8 : 4;
-        int const L = R / epl;
-        unsigned const blocks = (unsigned)( ( n_rows * L + 255 ) / 256 );
-        if ( epl == 8 )
-            launch_pos_epl<8, true>( L, blocks, n_rows, pos, coeff32, v.v32.get(), target, s, order );
-        else
-            launch_pos_epl<4, true>( L, blocks, n_rows, pos, coeff32, v.v32.get(), target, s, order );
-    }
-    else
-    {
-        int const L = R / 4;
-        unsigned const blocks = (unsigned)( ( n_rows * L + 255 ) / 256 );
-        launch_pos_epl<4, false>( L, blocks, n_rows, pos, coeff64, v.v64.get(), target, s, order );
-    }
-    check_launch( "k_apply_pos" );
+    if ( n_rows > 0 )
+        launch_pos<1>( n_rows, uniform_row, pos, coeff64, coeff32, v.v64.get(), v.v32.get(), target, 1, 0, s,
+                       order );
 }
 
 void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
@@ -361,6 +362,42 @@ void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *pos, double co
         return;
     SortedValues const v = permute_values( n_src, perm, values, coeff32 != nullptr, s );
     apply_pos( n_tgt, uniform_row, pos, coeff64, coeff32, v, target, s, order );
+}
+
+template <int CB>
+static void apply_fields( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
+                          float const *coeff32, uint32_t const *perm, FieldView in, FieldView out, int64_t c0,
+                          cudaStream_t s, uint32_t const *order )
+{
+    SortedValues v;
+    if ( coeff32 )
+        v.v32.allocate( std::max<int64_t>( 1, CB * in.n ), s );
+    else
+        v.v64.allocate( std::max<int64_t>( 1, CB * in.n ), s );
+    if ( in.n > 0 )
+    {
+        k_permute_fields<CB><<<(unsigned)( ( in.n + 255 ) / 256 ), 256, 0, s>>>( in, c0, perm, v.v64.get(),
+                                                                                v.v32.get() );
+        check_launch( "k_permute_fields" );
+    }
+    launch_pos<CB>( n_tgt, uniform_row, pos, coeff64, coeff32, v.v64.get(), v.v32.get(), out.wbase + c0 * out.cs,
+                    out.ps, out.cs, s, order );
+}
+
+void apply_sorted_multi( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
+                         float const *coeff32, uint32_t const *perm, FieldView in, FieldView out, cudaStream_t s,
+                         uint32_t const *order )
+{
+    if ( n_tgt == 0 )
+        return;
+    for ( int64_t c0 = 0; c0 < in.n_comp; c0 += 4 )
+    {
+        auto const run = in.n_comp - c0 >= 4   ? apply_fields<4>
+                         : in.n_comp - c0 == 3 ? apply_fields<3>
+                         : in.n_comp - c0 == 2 ? apply_fields<2>
+                                               : apply_fields<1>;
+        run( n_tgt, uniform_row, pos, coeff64, coeff32, perm, in, out, c0, s, order );
+    }
 }
 
 // uniform_row > 0: every row has that length (offset[i] = i * uniform_row);
@@ -428,13 +465,10 @@ void apply_csr( int64_t n_tgt, int32_t const *offset, int32_t const *idx, double
         return;
     bool const f32 = coeff32 != nullptr;
     void const *coeff = f32 ? (void const *)coeff32 : (void const *)coeff64;
-    if ( uniform_row > 0 && uniform_row % 4 == 0 && is_pow2( uniform_row / 4 ) &&
-         uniform_row / 4 <= 32 )
+    if ( !f32 && apply_sorted_supported( uniform_row ) )
     {
-        if ( f32 )
-            launch_vec<true>( uniform_row, n_tgt, idx, coeff, values, target, s );
-        else
-            launch_vec<false>( uniform_row, n_tgt, idx, coeff, values, target, s );
+        // (a saved operator has no positions: the same sums by index)
+        launch_pos<1>( n_tgt, uniform_row, idx, coeff64, nullptr, values, nullptr, target, 1, 0, s, nullptr );
         return;
     }
     int const len = uniform_row > 0 ? uniform_row : mean_row;

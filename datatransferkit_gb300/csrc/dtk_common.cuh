@@ -713,6 +713,10 @@ SortedValues permute_values( int64_t n_src, uint32_t const *perm, double const *
 // share most of their neighbours' values in L1) or in row order
 void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double const *coeff64, float const *coeff32,
                 SortedValues const &v, double *target, cudaStream_t s, uint32_t const *order = nullptr );
+// several components, up to four a pass
+void apply_sorted_multi( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
+                         float const *coeff32, uint32_t const *perm, FieldView in, FieldView out, cudaStream_t s,
+                         uint32_t const *order );
 void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
                    float const *coeff32, int64_t n_src, uint32_t const *perm, double const *values,
                    double *target, cudaStream_t s, uint32_t const *order = nullptr );
