@@ -5,7 +5,8 @@
 //  * up to 16k pairs one block sorts everything in shared memory, one launch
 //    for all digits (a create at 1k points 563 -> 417 us, at 10k 1228 -> 1043
 //    us against five launches a digit; 16 pairs a thread is what the block's
-//    registers and 160 KB of shared memory hold);
+//    registers and 160 KB of shared memory hold), with as many pairs a thread
+//    as n needs, two at a time (10k pairs, 30 bits: 16 pairs 56 us, 10 47);
 //  * beyond, a pass is a per-tile histogram and a stable scatter.  Every warp
 //    ranks its own run of the tile against its own counts (__match_any_sync
 //    for the lanes, a shared-memory count per digit and warp for the rounds),
@@ -125,6 +126,66 @@ __global__ void __launch_bounds__( SCAN_THREADS )
             out[base + i] = run;
         run += vals[i];
     }
+}
+
+// One block: the whole scan of a short array, SCAN_ONE_TILE values a round
+// (three launches of about 4 us each are mostly their latency: 12 -> 4 us at 1k
+// values, 13 -> 11 at 10k, two scans a tree).
+constexpr int SCAN_ONE_THREADS = 1024;
+constexpr int SCAN_ONE_TILE = SCAN_ONE_THREADS * SCAN_ITEMS;
+constexpr int64_t SCAN_ONE_MAX = 2 * SCAN_ONE_TILE;
+
+__global__ void __launch_bounds__( SCAN_ONE_THREADS )
+    k_scan_one( int64_t const *in, int64_t *out, int64_t n )
+{
+    __shared__ int64_t s_warp[SCAN_ONE_THREADS / 32];
+    int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t carry = 0;
+    for ( int64_t t = 0; t < n; t += SCAN_ONE_TILE )
+    {
+        int64_t const base = t + (int64_t)threadIdx.x * SCAN_ITEMS;
+        int64_t v[SCAN_ITEMS], sum = 0;
+#pragma unroll
+        for ( int i = 0; i < SCAN_ITEMS; ++i )
+        {
+            v[i] = base + i < n ? in[base + i] : 0;
+            sum += v[i];
+        }
+        int64_t incl = sum;
+#pragma unroll
+        for ( int o = 1; o < 32; o <<= 1 )
+        {
+            int64_t const x = __shfl_up_sync( 0xffffffffu, incl, o );
+            if ( lane >= o )
+                incl += x;
+        }
+        if ( lane == 31 )
+            s_warp[warp] = incl;
+        __syncthreads();
+        // every warp scans the warps' sums for itself
+        int64_t w = s_warp[lane];
+#pragma unroll
+        for ( int o = 1; o < 32; o <<= 1 )
+        {
+            int64_t const x = __shfl_up_sync( 0xffffffffu, w, o );
+            if ( lane >= o )
+                w += x;
+        }
+        int64_t const total = __shfl_sync( 0xffffffffu, w, 31 );
+        int64_t const before = __shfl_sync( 0xffffffffu, w, warp ? warp - 1 : 0 );
+        int64_t run = carry + ( warp ? before : 0 ) + incl - sum;
+#pragma unroll
+        for ( int i = 0; i < SCAN_ITEMS; ++i )
+        {
+            if ( base + i < n )
+                out[base + i] = run;
+            run += v[i];
+        }
+        carry += total;
+        __syncthreads();
+    }
+    if ( threadIdx.x == 0 )
+        out[n] = carry;
 }
 
 // ---------------------------------------------------------------------------
@@ -384,24 +445,20 @@ void launch_block_sort( uint32_t *keys, uint32_t *values, int64_t n, int bits, c
 
 void exclusive_scan_i64( int64_t const *in, int64_t *out, int64_t n, cudaStream_t s )
 {
-    int64_t const n_tiles = std::max<int64_t>( 1, ( n + SCAN_TILE - 1 ) / SCAN_TILE );
+    if ( n <= SCAN_ONE_MAX )
+    {
+        k_scan_one<<<1, SCAN_ONE_THREADS, 0, s>>>( in, out, n );
+        check_launch( "k_scan_one" );
+        return;
+    }
+    int64_t const n_tiles = ( n + SCAN_TILE - 1 ) / SCAN_TILE;
     DeviceBuffer<int64_t> sums( n_tiles + 1, s );
-    if ( n > 0 )
-    {
-        k_tile_reduce<<<(unsigned)n_tiles, SCAN_THREADS, 0, s>>>( in, n, sums.get() );
-        check_launch( "k_tile_reduce" );
-    }
-    else
-    {
-        DTK_CUDA_OR_THROW( cudaMemsetAsync( sums.get(), 0, sizeof( int64_t ), s ) );
-    }
-    k_scan_tile_sums<<<1, SCAN_THREADS, 0, s>>>( sums.get(), n > 0 ? n_tiles : 1, out + n );
+    k_tile_reduce<<<(unsigned)n_tiles, SCAN_THREADS, 0, s>>>( in, n, sums.get() );
+    check_launch( "k_tile_reduce" );
+    k_scan_tile_sums<<<1, SCAN_THREADS, 0, s>>>( sums.get(), n_tiles, out + n );
     check_launch( "k_scan_tile_sums" );
-    if ( n > 0 )
-    {
-        k_tile_scan<<<(unsigned)n_tiles, SCAN_THREADS, 0, s>>>( in, out, n, sums.get() );
-        check_launch( "k_tile_scan" );
-    }
+    k_tile_scan<<<(unsigned)n_tiles, SCAN_THREADS, 0, s>>>( in, out, n, sums.get() );
+    check_launch( "k_tile_scan" );
 }
 
 void radix_sort_pairs( uint32_t *keys, uint32_t *values, int64_t n, int bits,
@@ -411,12 +468,17 @@ void radix_sort_pairs( uint32_t *keys, uint32_t *values, int64_t n, int bits,
         return;
     if ( n <= RB_THREADS * RB_MAX_ROUNDS )
     {
-        if ( n <= RB_THREADS * 2 )
-            launch_block_sort<2>( keys, values, n, bits, s );
-        else if ( n <= RB_THREADS * 6 )
-            launch_block_sort<6>( keys, values, n, bits, s );
-        else
-            launch_block_sort<RB_MAX_ROUNDS>( keys, values, n, bits, s );
+        switch ( ( n + 2 * RB_THREADS - 1 ) / ( 2 * RB_THREADS ) )
+        {
+        case 1: launch_block_sort<2>( keys, values, n, bits, s ); break;
+        case 2: launch_block_sort<4>( keys, values, n, bits, s ); break;
+        case 3: launch_block_sort<6>( keys, values, n, bits, s ); break;
+        case 4: launch_block_sort<8>( keys, values, n, bits, s ); break;
+        case 5: launch_block_sort<10>( keys, values, n, bits, s ); break;
+        case 6: launch_block_sort<12>( keys, values, n, bits, s ); break;
+        case 7: launch_block_sort<14>( keys, values, n, bits, s ); break;
+        default: launch_block_sort<RB_MAX_ROUNDS>( keys, values, n, bits, s ); break;
+        }
         return;
     }
     int64_t const n_tiles = ( n + RS_TILE - 1 ) / RS_TILE;

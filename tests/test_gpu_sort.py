@@ -1,5 +1,5 @@
-"""The point sort at the edges of its paths (one block up to 2 / 6 / 16 pairs a
-thread of 1024, tiles of 4096 pairs with summed or scanned histograms): a
+"""The point sort at the edges of its paths (one block, an even number of pairs a
+thread of 1024 up to 16, tiles of 4096 pairs with summed or scanned histograms): a
 search over n sources and n targets visits every point of both sorted orders,
 so a lost, doubled or misplaced pair changes its rows.  Rows are bit-exact."""
 import numpy as np
@@ -13,7 +13,8 @@ from oracle import cpu
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [2, 33, 2048, 2049, 6144, 6145, 16384, 16385, 128 * 4096, 128 * 4096 + 1])
+@pytest.mark.parametrize("n", [2, 33, 2048, 2049, 4097, 6144, 6145, 8193, 10241, 12289, 14337, 16384, 16385,
+                                128 * 4096, 128 * 4096 + 1])
 def test_sorted_orders_at_path_edges(n):
     src, tgt = syn.uniform_points(n, 31), syn.uniform_points(n, 32)
     src[n // 2:] = src[: n - n // 2]  # equal keys: a stable order is part of the result
