@@ -42,7 +42,8 @@ constexpr int FX_DIGIT = 29;
 constexpr int FX_MASK = ( 1 << FX_DIGIT ) - 1, FX_HALF = 1 << ( FX_DIGIT - 1 );
 constexpr int FX_ONE = 60;  // the two leading digits as an integer: 2^60 is 1
 constexpr int FX_COEF = 58; // rotation factors: 2^58 is 1
-constexpr int FX_V = 54;    // column 0 of V (two digits): 2^54 is 1 at row 0's scale (headroom 64)
+constexpr int FX_V = 54;    // column 0 of V (two digits): 2^54 is 1 at row 0's scale (headroom 64, eight times that after each fx_shrink_v)
+constexpr int FX_V_SHRINK = 18; // by how much the unit may grow (rows 2^-18 of row 0's scale)
 constexpr int FX_LOG = 224;    // rotations (a quadratic basis takes 113 on a fine cloud, up to 183 at unit spacing)
 constexpr int FX_NOISE = 16;   // off-diagonal entries up to 16 units of the last digit count as zero
 constexpr int FX_MAX_EXP = 40; // scales 2^-40 .. 2^40, so that FP32 holds every squared magnitude that decides
@@ -540,6 +541,21 @@ __host__ __device__ __noinline__ bool fx_exact_go( State const st )
     return sqrt( 2.0 * acc ) > 2.220446049250313e-16;
 }
 
+// V in units eight times as large (an entry outgrew its leading digit: rows
+// whose scale is far below row 0's; 10 of 600k matrices of 20 neighbours, 58
+// of 100k of 15, and one matrix left to the FP64 kernel takes its 1 ms).
+template <int M, class State>
+__host__ __device__ __forceinline__ void fx_shrink_v( State const &st )
+{
+#pragma unroll 1
+    for ( int k = 0; k < M; ++k )
+    {
+        FxNum<2> const v = st.v( k );
+        int64_t const x = ( (int64_t)v.d[0] * ( int64_t( 1 ) << FX_DIGIT ) ) + v.d[1];
+        st.set_v( k, fx_num<2>( ( x + 4 ) >> 3 ) );
+    }
+}
+
 // Runs the Jacobi on the state (live: this lane's matrix takes part), all
 // lanes of the warp together; returns the rotations made, or -1 when the
 // matrix is handed back.
@@ -548,6 +564,7 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
 {
     using Lay = FxLayout<M>;
     int const d0 = live ? st.exp( 0 ) : 0; // V's unit
+    int fv = FX_V;                         // 2^fv is 1 in it
     int it = 0;
     bool ok = live;
     while ( st.any( live ) )
@@ -649,10 +666,20 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
                 if ( h == 0 )
                 {
                     // column 0 of V
-                    FxNum<2> const a = st.v( swap ? q : p ), b = st.v( swap ? p : q );
+                    FxNum<2> a = st.v( swap ? q : p ), b = st.v( swap ? p : q );
                     bool fx, fy;
-                    st.set_v( p, fx_dot( r.cx, a, r.sx, b, fx ) );
-                    st.set_v( q, fx_dot( r.cy, b, r.sy_neg, a, fy ) );
+                    FxNum<2> vp = fx_dot( r.cx, a, r.sx, b, fx ), vq = fx_dot( r.cy, b, r.sy_neg, a, fy );
+                    while ( !( fx && fy ) && fv > FX_V - FX_V_SHRINK )
+                    {
+                        fx_shrink_v<M>( st );
+                        fv -= 3;
+                        a = st.v( swap ? q : p );
+                        b = st.v( swap ? p : q );
+                        vp = fx_dot( r.cx, a, r.sx, b, fx );
+                        vq = fx_dot( r.cy, b, r.sy_neg, a, fy );
+                    }
+                    st.set_v( p, vp );
+                    st.set_v( q, vq );
                     fits = fx && fy;
                 }
                 else
@@ -677,6 +704,13 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
         ok = turn ? live : ok;
         st.sync();
     }
+    {
+        // (the lane that turned V knows its unit)
+        int shrunk = FX_V - fv, none = 0;
+        float zero = 0.f;
+        st.merge( shrunk, none, zero );
+        fv = FX_V - shrunk;
+    }
     // w_k = v_k / E(k, k)
     st.for_parts( [&]( int h ) {
 #pragma unroll 1
@@ -693,7 +727,7 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
                 int z;
                 bool negative;
                 uint64_t const m = fx_normal( v, z, negative );
-                w = fx_double( m, d - d0 - z - FX_V, negative ) / fx_double( (uint64_t)f, 2 * d - FX_ONE, false );
+                w = fx_double( m, d - d0 - z - fv, negative ) / fx_double( (uint64_t)f, 2 * d - FX_ONE, false );
             }
             st.w( k ) = w;
         }

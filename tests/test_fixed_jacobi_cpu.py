@@ -105,3 +105,19 @@ def test_more_rotations_than_the_cap_are_handed_back(fixed):
     off, idx, _ = cpu.knn(src, tgt, 32)
     _, back = fixed(moments_of(src, tgt, idx, 32, 1, 2), 10, cap=40)
     assert back.all()
+
+
+def test_rows_far_below_row_0_s_scale(fixed):
+    # half as many neighbours again as the basis has: V outgrows its first unit
+    src, tgt = syn.uniform_points(10000, 13), syn.uniform_points(10000, 14)
+    off, idx, _ = cpu.knn(src, tgt, 15)
+    got, back = fixed(moments_of(src, tgt, idx, 15, 2, 2), 10)
+    assert not back.any()
+    ref, other = both_oracles(src, tgt, off, idx, 2, 2)
+    deg = np.array([0, 1, 1, 1, 2, 2, 2, 2, 2, 2])
+    h = (15 / 10000) ** (1 / 3)
+    size = np.abs(ref * h ** deg).max(1)
+    err = np.abs((got - ref) * h ** deg).max(1) / size
+    spread = np.abs((other - ref) * h ** deg).max(1) / size
+    assert err.max() <= max(1e-12, 10 * spread.max())
+    assert np.sqrt(np.mean(err ** 2)) <= max(1e-12, 10 * np.sqrt(np.mean(spread ** 2)))

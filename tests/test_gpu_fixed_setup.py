@@ -40,7 +40,7 @@ def test_partial_warps(n_tgt, basis, rbf, k):
     check(syn.uniform_points(3000, 31), syn.uniform_points(n_tgt, 32), basis, rbf, k)
 
 
-@pytest.mark.parametrize("basis, k", [(2, 32), (1, 8)])
+@pytest.mark.parametrize("basis, k", [(2, 32), (1, 8), (2, 15)])  # (15: V in larger units)
 def test_both_layouts_give_the_same_bits(basis, k):
     src, tgt = syn.uniform_points(20000, 33), syn.uniform_points(40001, 34)
     whole = coefficients(src, tgt, basis, dtk.Wendland(4), k)[2].reshape(-1, k)  # one lane a matrix
