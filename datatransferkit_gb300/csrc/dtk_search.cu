@@ -1079,6 +1079,7 @@ struct KnnChunks
     int64_t n_big;
     unsigned *next;
     unsigned const *n_listed;
+    float const *bounds; // of a list: a guess of every query's k-th squared distance
 };
 
 __device__ __forceinline__ void chunk_range( KnnChunks const &ch, unsigned c, int64_t &w0, int64_t &len )
@@ -1307,7 +1308,10 @@ __global__ void __launch_bounds__( Q_WARPS * 32, KNN_BLOCKS_PER_SM )
     // beyond it are skipped as if the list were already that tight.  A query
     // that scans its chunk's leaf list skips every leaf beyond the list's
     // bound as well.
-    float spec = seeded && row == k ? next_spec : __int_as_float( 0x7f800000 );
+    float spec = row != k    ? __int_as_float( 0x7f800000 )
+                 : seeded    ? next_spec
+                 : ch.bounds ? __ldg( ch.bounds + w )
+                             : __int_as_float( 0x7f800000 );
     bool list_pass = !GROUPED && !head && row == k && s_nlist[wib] >= 0;
     if ( list_pass )
         spec = fminf( spec, s_list_r2[wib] );
@@ -1915,8 +1919,7 @@ template <int CAP>
 __global__ void __launch_bounds__( KL_THREADS, CAP == KL_CAP_SHORT ? KL_BLOCKS_SHORT : KL_BLOCKS )
     k_knn_lanes( TreeView tr, PointsView tgt, uint32_t const *order, int row, int per_warp, unsigned *next_chunk,
                  int64_t pilot_stride, float growth, int32_t const *offset, int32_t *idx_out, int32_t *pos_out,
-                 uint32_t *list,
-                 unsigned *n_listed, unsigned *status )
+                 uint32_t *list, float *list_bounds, unsigned *n_listed, unsigned *status )
 {
     unsigned *const n_failed = n_listed + 1, *const n_settled = n_listed + 2; // batches
     constexpr int UNROLL = KL_UNROLL;
@@ -1972,14 +1975,17 @@ __global__ void __launch_bounds__( KL_THREADS, CAP == KL_CAP_SHORT ? KL_BLOCKS_S
         int const n_real = tgt.n - w0 < 32 ? (int)( tgt.n - w0 ) : 32;
         int64_t const w = w0 + ( lane < n_real ? lane : n_real - 1 );
         int const qi = order ? (int)order[w] : (int)w;
-        auto pass_on = [&]( bool mine ) {
+        auto pass_on = [&]( bool mine, float bound ) {
             unsigned const m = __ballot_sync( FULL, mine );
             unsigned at = 0;
             if ( lane == 0 && m && !pilot_stride )
                 at = atomicAdd( n_listed, (unsigned)__popc( m ) );
             at = __shfl_sync( FULL, at, 0 );
             if ( mine && !pilot_stride )
+            {
                 list[at + __popc( m & lt_mask )] = (uint32_t)qi;
+                list_bounds[at + __popc( m & lt_mask )] = bound;
+            }
             return __popc( m );
         };
         if ( skipped < skip )
@@ -1992,7 +1998,10 @@ __global__ void __launch_bounds__( KL_THREADS, CAP == KL_CAP_SHORT ? KL_BLOCKS_S
                 at = atomicAdd( n_listed, (unsigned)( end - w0 ) );
             at = __shfl_sync( FULL, at, 0 );
             for ( int64_t i = w0 + lane; i < end; i += 32 )
+            {
                 list[at + (unsigned)( i - w0 )] = order ? order[i] : (uint32_t)i;
+                list_bounds[at + (unsigned)( i - w0 )] = inf;
+            }
             skipped += (int)run;
             batch += run - 1;
             continue;
@@ -2358,7 +2367,8 @@ __global__ void __launch_bounds__( KL_THREADS, CAP == KL_CAP_SHORT ? KL_BLOCKS_S
             __syncwarp();
             todo = __ballot_sync( FULL, !fin && !give_up );
         }
-        bool const failed = pass_on( give_up ) > n_real / 2;
+        // (the general kernel proves its bound or searches again)
+        bool const failed = pass_on( give_up, T > 0.f ? T : inf ) > n_real / 2;
         skip = failed ? min( 2 * skip + 1, 15 ) : 0;
         skipped = 0;
         if ( lane == 0 )
@@ -2762,25 +2772,26 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
         float const growth = (float)std::pow( std::min( 2.0, 0.7 * cap / row ), 2.0 / 3.0 );
         int const per_warp = (int)std::min<int64_t>( 16, std::max<int64_t>( 1, tgt.n / 32 / ( 4 * lane_warps ) ) );
         DeviceBuffer<uint32_t> list( tgt.n, s );
+        DeviceBuffer<float> bounds( tgt.n, s );
         auto const kernel = row <= 16 ? k_knn_lanes<KL_CAP_SHORT> : k_knn_lanes<KL_CAP>;
         int64_t const batches = ( tgt.n + 31 ) / 32;
         kernel<<<KL_PILOT / KL_WARPS, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, 1, next.get() + 1,
                                                            batches / KL_PILOT, growth, offset, idx, pos, list.get(),
-                                                           next.get() + 2, status );
+                                                           bounds.get(), next.get() + 2, status );
         check_launch( "k_knn_lanes(pilot)" );
         kernel<<<lane_blocks, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, per_warp, next.get() + 1, 0,
-                                                   growth, offset, idx, pos, list.get(), next.get() + 2, status );
+                                                   growth, offset, idx, pos, list.get(), bounds.get(), next.get() + 2, status );
         check_launch( "k_knn_lanes" );
         // what it left
         k_query_frame<<<8 * num_sms(), 256, 0, s>>>( tgt, list.get(), tree.scene.get(), qrec.get(), next.get() + 2 );
         check_launch( "k_query_frame" );
-        KnnChunks const rest{Q_SEQ, 0, next.get(), next.get() + 2};
+        KnnChunks const rest{Q_SEQ, 0, next.get(), next.get() + 2, bounds.get()};
         k_knn<false><<<num_sms() * KNN_BLOCKS_PER_SM, Q_WARPS * 32, 0, s>>>(
             view_of( tree ), tgt, list.get(), qrec.get(), k, rest, gv, offset, idx, pos, status );
         check_launch( "k_knn" );
         return;
     }
-    KnnChunks const ch{seq, n_big, next.get(), nullptr};
+    KnnChunks const ch{seq, n_big, next.get(), nullptr, nullptr};
     k_query_frame<<<blocks_for( tgt.n, 256 ), 256, 0, s>>>( tgt, order, tree.scene.get(), qrec.get() );
     check_launch( "k_query_frame" );
     if ( groups.tgt_grp )
