@@ -1079,7 +1079,11 @@ struct KnnChunks
     int64_t n_big;
     unsigned *next;
     unsigned const *n_listed;
-    float const *bounds; // of a list: a guess of every query's k-th squared distance
+    // Of a list, per query: a guess of its k-th squared distance, +inf for a
+    // query next to the one before it in the targets' order, which seeds it,
+    // or -1 (no guess).  Unrelated queries do not seed each other: a list of
+    // far neighbours is a bound that prunes nothing near.
+    float const *bounds;
 };
 
 __device__ __forceinline__ void chunk_range( KnnChunks const &ch, unsigned c, int64_t &w0, int64_t &len )
@@ -1256,7 +1260,9 @@ __global__ void __launch_bounds__( Q_WARPS * 32, KNN_BLOCKS_PER_SM )
             __ldg( reinterpret_cast<uint32_t const *>( qrec + w ) + lane );
     __syncwarp();
     Query const &q = s_query[wib];
-    bool const seeded = prev_row == row && ( !GROUPED || prev_g == rg.g );
+    float const guess = ch.bounds ? __ldg( ch.bounds + w ) : __int_as_float( 0x7f800000 );
+    bool const seeded =
+        prev_row == row && ( !GROUPED || prev_g == rg.g ) && !( guess < __int_as_float( 0x7f800000 ) );
 
     if ( seeded )
     {
@@ -1308,10 +1314,9 @@ __global__ void __launch_bounds__( Q_WARPS * 32, KNN_BLOCKS_PER_SM )
     // beyond it are skipped as if the list were already that tight.  A query
     // that scans its chunk's leaf list skips every leaf beyond the list's
     // bound as well.
-    float spec = row != k    ? __int_as_float( 0x7f800000 )
-                 : seeded    ? next_spec
-                 : ch.bounds ? __ldg( ch.bounds + w )
-                             : __int_as_float( 0x7f800000 );
+    float spec = row != k ? __int_as_float( 0x7f800000 ) : seeded ? next_spec : guess;
+    if ( spec < 0.f )
+        spec = __int_as_float( 0x7f800000 );
     bool list_pass = !GROUPED && !head && row == k && s_nlist[wib] >= 0;
     if ( list_pass )
         spec = fminf( spec, s_list_r2[wib] );
@@ -2000,7 +2005,7 @@ __global__ void __launch_bounds__( KL_THREADS, CAP == KL_CAP_SHORT ? KL_BLOCKS_S
             for ( int64_t i = w0 + lane; i < end; i += 32 )
             {
                 list[at + (unsigned)( i - w0 )] = order ? order[i] : (uint32_t)i;
-                list_bounds[at + (unsigned)( i - w0 )] = inf;
+                list_bounds[at + (unsigned)( i - w0 )] = i == w0 ? -1.f : inf;
             }
             skipped += (int)run;
             batch += run - 1;
@@ -2036,7 +2041,8 @@ __global__ void __launch_bounds__( KL_THREADS, CAP == KL_CAP_SHORT ? KL_BLOCKS_S
         };
         auto position = [&]( uint32_t v ) { return s_range[wib][( v >> 5 ) & 127u].x + (int)( v & 31u ); };
         unsigned todo = __ballot_sync( FULL, !fin ), sub = 0;
-        for ( int round = 0; todo; ++round )
+        int rounds = 0;
+        for ( int round = 0; todo; ++round, ++rounds )
         {
             // the lanes searched together (a split leaves a part of them in sub)
             sub &= todo;
@@ -2368,11 +2374,12 @@ __global__ void __launch_bounds__( KL_THREADS, CAP == KL_CAP_SHORT ? KL_BLOCKS_S
             todo = __ballot_sync( FULL, !fin && !give_up );
         }
         // (the general kernel proves its bound or searches again)
-        bool const failed = pass_on( give_up, T > 0.f ? T : inf ) > n_real / 2;
+        int const left = pass_on( give_up, T > 0.f && T < inf ? T : -1.f );
+        bool const failed = left > n_real / 2;
         skip = failed ? min( 2 * skip + 1, 15 ) : 0;
         skipped = 0;
         if ( lane == 0 )
-            atomicAdd( failed ? n_failed : n_settled, 1u );
+            atomicAdd( failed || rounds > 5 || ( pilot_stride && left > n_real / 4 ) ? n_failed : n_settled, 1u );
         float sum = kth < inf ? kth : 0.f;
         int const got = __popc( __ballot_sync( FULL, kth < inf ) );
 #pragma unroll
@@ -2758,8 +2765,9 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
     // Search with the tree, k_knn alone against this: k = 8, 800k targets 1.97
     // / 1.73 ms, 2M 4.28 / 3.10, 8M 15.2 / 9.6; k = 20, 2M 4.39 / 4.00 (1M 2.46
     // / 2.31), 8M 15.6 / 13.1; k = 32, 1M 2.77 / 2.93, 2M 5.01 / 4.89, 8M 17.5
-    // / 16.1.  At 3M and k = 20: grid 7.5 / 6.9, sphere 5.5 / 5.1, clusters 6.8
-    // / 7.1, duplicates 10.1 / 9.5, targets far outside 5.6 / 5.6.
+    // / 15.8.  At 3M and k = 20: grid 7.5 / 6.9, sphere 5.5 / 5.1, clusters 6.8
+    // / 7.2, duplicates 10.1 / 9.6, targets far outside 5.6 / 5.7, coordinates
+    // to the fourth power 14.2 / 15.4.
     int const row = (int)std::min<int64_t>( k, tree.n );
     int const lane_blocks = num_sms() * ( row <= 16 ? KL_BLOCKS_SHORT : KL_BLOCKS );
     int64_t const lane_warps = (int64_t)lane_blocks * KL_WARPS;
