@@ -704,10 +704,10 @@ def run_ours(args, rank, world, local_rank):
     traffic_pt = read_profile_traffic("setup_mixed_traffic.txt", "bytes_per_target")
     traffic_q = read_profile_traffic("knn_traffic.txt", "bytes_per_query")
     instr_q = read_profile_traffic("knn_traffic.txt", "warp_instructions_per_query")
-    # kNN query launch, algorithmic bytes: per query its 64-byte record, k
+    # kNN query launch, algorithmic bytes: per query its point and place, k
     # indices and k sorted positions out and the offset; per source its FP64 +
     # FP32 sorted copies and its index
-    q_bytes = n_tgt * (64 + 8 * k + 4) + len(src) * (24 + 12 + 4)
+    q_bytes = n_tgt * (24 + 4 + 8 * k + 4) + len(src) * (24 + 12 + 4)
     q_gbs = q_bytes / (query_ms / 1e3) / 1e9
     # the issue ruler: warp instructions (ncu count per query) over the SMs'
     # issue rate, one warp instruction per cycle per scheduler at the sampled clock
@@ -742,7 +742,7 @@ def run_ours(args, rank, world, local_rank):
         "e2e": {"value": total_targets / (ms_e2e / 1e3), "unit": UNIT,
                 "h2d_bytes_per_step": int(src_h.numel() * 8 + tgt_h.numel() * 8 + val_h.numel() * 8),
                 "d2h_bytes_per_step": int(out_h.numel() * 8)},
-        "roofline": {"bound": "hbm", "kernel": "k_knn", "achieved": q_gbs, "peak": hbm, "unit": "GB/s",
+        "roofline": {"bound": "hbm", "kernel": "k_knn_lanes", "achieved": q_gbs, "peak": hbm, "unit": "GB/s",
                      "frac": q_gbs / hbm, "traffic": (traffic_q * n_tgt) if traffic_q else None,
                      "launch_ms": query_ms, "issue_frac": issue_frac},
         "cpu_baseline": ({"value": cpu_value, "unit": UNIT, "cores": cpu["threads"], "kind": "port",
@@ -759,7 +759,8 @@ def run_ours(args, rank, world, local_rank):
     detail.update({
         "roofline_detail": {
             "peak_source": hbm_src, "algorithmic_bytes": q_bytes,
-            "note": ("the dominant kernel of a mixed step; algorithmic bytes = N_t (64 + 8k + 4) "
+            "note": ("the dominant kernel of a mixed step (launch_ms: pilot, search and the queries left to "
+                     "k_knn); algorithmic bytes = N_t (24 + 4 + 8k + 4) "
                      "+ N_s (24 + 12 + 4); traffic = the ncu DRAM bytes per query of profiles/knn_traffic.txt "
                      "x N_t; issue_frac = ncu warp instructions per query x N_t / launch time / "
                      "(SMs x 4 schedulers x sampled SM clock)")},
