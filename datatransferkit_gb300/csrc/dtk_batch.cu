@@ -8,13 +8,15 @@
 // processed in problem-major Morton order.  The setup is planned on the
 // device: a stable key sort splits the processing order into buckets of
 // (basis, rbf, path), and a layout kernel cuts the buckets into tasks of 32
-// targets (longest rows first).  One persistent launch runs every task: a
+// targets (longest rows first).  One persistent launch runs every task
+// (k_batch_fixed, the Jacobi in fixed point; a second one the Buhmann weights
+// and what that form hands back, with the FP64 Jacobi): a
 // warp gathers its targets' rows with G lanes a target (1 for kNN rows, the
 // single operator's arithmetic; for radius rows, 0 to thousands of entries,
 // G is tuned by timing candidates on a sample of the tasks at create), then
 // runs the reference Jacobi one target a lane.  Mixed-form kNN rows run the
 // fused mixed kernel per bucket instead.  The plan is kept: a re-setup on
-// new coordinates with the same rows is the persistent launch alone,
+// new coordinates with the same rows is the persistent launches alone,
 // captured into a CUDA graph and replayed.
 //
 // Apply is one persistent launch over a schedule of warp tasks.  Rows are

@@ -14,7 +14,11 @@
 // children of a node at once; each wide node also keeps its Morton cell (an
 // inset FP32 box) and its parent.
 //
-// kNN query: a warp runs chunks of 48 Morton-consecutive targets one after
+// kNN query: three kernels give the same rows: k_nearest (k = 1, a lane a
+// query), k_knn_lanes (large target sets, 32 queries a warp) and k_knn (the
+// rest, batches of problems, and what k_knn_lanes leaves), a warp a query.
+//
+// k_knn: a warp runs chunks of 48 Morton-consecutive targets one after
 // the other, taking the next chunk from a counter; the k best (d2, index)
 // keys sit one per lane, sorted across lanes.
 // The first target of a chunk starts from the 32 Morton-sorted sources around
@@ -2613,10 +2617,9 @@ void build_lbvh( PointsView src, Lbvh &tree, unsigned *status, cudaStream_t s,
                                                                  range_hi.get(), tree.nodes.get() );
         check_launch( "k_pack_children" );
     }
-    k_refit<<<blocks_for( nl, REFIT_THREADS / REFIT_LANES ), REFIT_THREADS, 0, s>>>( tree.f4.get(), tree.leaf_start.get(), nl,
-                                                     left.get(), right.get(), parent_node.get(),
-                                                     parent_leaf.get(), tree.nodes.get(), flags.get(),
-                                                     tree.root_box.get(), status );
+    k_refit<<<blocks_for( nl, REFIT_THREADS / REFIT_LANES ), REFIT_THREADS, 0, s>>>(
+        tree.f4.get(), tree.leaf_start.get(), nl, left.get(), right.get(), parent_node.get(), parent_leaf.get(),
+        tree.nodes.get(), flags.get(), tree.root_box.get(), status );
     check_launch( "k_refit" );
     tree.n_wide = 0;
     if ( ni > 0 )
@@ -2788,7 +2791,8 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
                                                            bounds.get(), next.get() + 2, status );
         check_launch( "k_knn_lanes(pilot)" );
         kernel<<<lane_blocks, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, per_warp, next.get() + 1, 0,
-                                                   growth, offset, idx, pos, list.get(), bounds.get(), next.get() + 2, status );
+                                                   growth, offset, idx, pos, list.get(), bounds.get(), next.get() + 2,
+                                                   status );
         check_launch( "k_knn_lanes" );
         // what it left
         k_query_frame<<<8 * num_sms(), 256, 0, s>>>( tgt, list.get(), tree.scene.get(), qrec.get(), next.get() + 2 );
