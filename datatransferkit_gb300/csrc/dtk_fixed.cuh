@@ -307,10 +307,14 @@ __host__ __device__ __forceinline__ FxRotation fx_rotation( int64_t fl, int64_t 
     int const u = dl > ds ? dl : ds; // common unit 2^(2u - 60)
     int const hl = u - dl, hs = u - ds;
     uint64_t const x0 = fx_shr( (uint64_t)fl, 2 * hl ) - fx_shr( (uint64_t)fs, 2 * hs );
-    uint64_t const y0 = fx_shr( bm << 1, zb + hl + hs ); // 2 |b|
-    // both below 2^63 with the larger one's leading bit there
-    int const z = fx_clz( x0 | y0 ) - 1;
-    uint64_t const x = x0 << ( z & 63 ), y = y0 << ( z & 63 );
+    int const sh = zb + hl + hs; // 2 |b| = (bm << 1) 2^-sh
+    // x0 and 2 |b| scaled by 2^z, below 2^63 with the larger one's leading bit
+    // there.  2 |b| comes from bm, not from its whole units: with a difference
+    // of a few units (nearly equal diagonal entries, as grids give them) what
+    // is cut off there is the angle, and c and s no longer belong together.
+    int const zx = fx_clz( x0 ) - 1;
+    int const z = x0 && zx < sh - 1 ? zx : sh - 1;
+    uint64_t const x = x0 ? x0 << ( z & 63 ) : 0, y = fx_shr( bm << 1, sh - z );
     uint64_t const r2 = fx_mulhi( x, x ) + fx_mulhi( y, y ); // about [2^60, 2^63)
     int const h = r2 < ( 1ull << 62 ) ? 1 : 0;               // sqrt of the scaling
     uint64_t const g = fx_inv_sqrt( r2 << ( 2 * h ) );       // 2^64 / r = g 2^h / 2^62
