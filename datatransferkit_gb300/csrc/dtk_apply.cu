@@ -97,10 +97,12 @@ bool is_pow2( int v ) { return v > 0 && ( v & ( v - 1 ) ) == 0; }
 // it (64 cycles an instruction a warp): one FMA an entry, and the lanes' partial
 // sums of a row are added for as many rows as there are lanes at once, each
 // lane ending with one row (2M rows of 32 with the permutation 257 -> 201 us,
-// 118 us of them the bytes).  A field of several
-// components keeps a point's components side by side, up to four a pass, so
-// that positions and coefficients are read once (three components of 1M rows of
-// 32, mixed: 480 -> 143 us against FP64 sums by index).  Rows go in
+// 118 us of them the bytes).  A field of several components keeps a point's
+// components side by side, up to four a pass, so that positions and
+// coefficients are read once.  Its sums are FP64 in both forms (a double-float
+// has FP32's range and 48 bits); FP32 coefficients are widened on the integer
+// pipe.  Three components of 1M rows of 32, mixed: 480 us by index, 202 us so,
+// 269 with the conversions on the FP64 pipe.  Rows go in
 // the targets' Morton order when the operator has it, so that consecutive
 // rows share most of their neighbours' values in L1 (0.70 -> 0.59 ms for 8M
 // rows of 32; 16 entries a lane instead of 8 was 1.26 ms, 4 no different).
@@ -166,20 +168,55 @@ __device__ __forceinline__ double df_group_sum( float s, float cs )
     return (double)s + (double)cs;
 }
 
-// Mixed form: L lanes per row, each lane EPL consecutive entries (EPL a
-// multiple of 4), CB components.
-template <int L, int EPL, int CB>
+// Exactly (double)c on the integer pipe: a conversion takes the FP64 pipe 64
+// cycles a warp, as an FMA does, and where a condition turns it off as well.
+__device__ __forceinline__ double widen( float c )
+{
+    unsigned const e = __float_as_uint( c ) & 0x7f800000u;
+    // the exponent's bias 127 -> 1023; a subnormal is made normal first, 2^24
+    // times as large, and an infinity or NaN goes to the largest exponent
+    unsigned bias = 896u << 20;
+    if ( e == 0u || e == 0x7f800000u )
+    {
+        bias = c == 0.f ? 0u : e ? 1792u << 20 : 872u << 20;
+        c = e ? c : __fmul_rn( c, 16777216.f );
+    }
+    unsigned const b = __float_as_uint( c );
+    return __hiloint2double( (int)( ( b & 0x80000000u ) | ( ( ( b & 0x7fffffffu ) >> 3 ) + bias ) ), (int)( b << 29 ) );
+}
+
+// Four consecutive coefficients as doubles.
+__device__ __forceinline__ void load_coeff4( double const *p, double *c )
+{
+    double2 const c0 = __ldcs( reinterpret_cast<double2 const *>( p ) );
+    double2 const c1 = __ldcs( reinterpret_cast<double2 const *>( p + 2 ) );
+    c[0] = c0.x;
+    c[1] = c0.y;
+    c[2] = c1.x;
+    c[3] = c1.y;
+}
+__device__ __forceinline__ void load_coeff4( float const *p, double *c )
+{
+    float4 const v = __ldcs( reinterpret_cast<float4 const *>( p ) );
+    c[0] = widen( v.x );
+    c[1] = widen( v.y );
+    c[2] = widen( v.z );
+    c[3] = widen( v.w );
+}
+
+// Mixed form, one component: L lanes per row, each lane EPL consecutive entries
+// (EPL a multiple of 4).
+template <int L, int EPL>
 __global__ void __launch_bounds__( 256 )
     k_apply_pos( int64_t n_tgt, int32_t const *__restrict__ pos, float const *__restrict__ coeff,
-                 float2 const *__restrict__ sorted, double *__restrict__ target, int64_t ps, int64_t cs_out,
-                 uint32_t const *__restrict__ order )
+                 float2 const *__restrict__ sorted, double *__restrict__ target, uint32_t const *__restrict__ order )
 {
     constexpr int R = EPL * L;
     int64_t const gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int64_t const row0 = gt / L;
     int64_t const row = ( order && row0 < n_tgt ) ? (int64_t)__ldg( order + row0 ) : row0;
     int const sub = (int)( gt % L );
-    float s[CB] = {}, cs[CB] = {};
+    float s = 0.f, cs = 0.f;
     if ( row < n_tgt )
     {
 #pragma unroll
@@ -188,32 +225,24 @@ __global__ void __launch_bounds__( 256 )
             int64_t const e = row * R + EPL * sub + q;
             int4 const ix = __ldcs( reinterpret_cast<int4 const *>( pos + e ) );
             float4 const c = __ldcs( reinterpret_cast<float4 const *>( coeff + e ) );
-            int const at[4] = {ix.x, ix.y, ix.z, ix.w};
-            float const cj[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-            for ( int j = 0; j < 4; ++j )
-            {
-                float2 const *v = sorted + (int64_t)CB * at[j];
-#pragma unroll
-                for ( int k = 0; k < CB; ++k )
-                    df_axpy( cj[j], __ldg( v + k ), s[k], cs[k] );
-            }
+            df_axpy( c.x, __ldg( sorted + ix.x ), s, cs );
+            df_axpy( c.y, __ldg( sorted + ix.y ), s, cs );
+            df_axpy( c.z, __ldg( sorted + ix.z ), s, cs );
+            df_axpy( c.w, __ldg( sorted + ix.w ), s, cs );
         }
     }
-#pragma unroll
-    for ( int k = 0; k < CB; ++k )
-    {
-        double const sum = df_group_sum<L>( s[k], cs[k] );
-        if ( row < n_tgt && sub == 0 )
-            target[row * ps + k * cs_out] = sum;
-    }
+    double const sum = df_group_sum<L>( s, cs );
+    if ( row < n_tgt && sub == 0 )
+        target[row] = sum;
 }
 
-// FP64 form: L lanes take L rows, each lane EPL consecutive entries of every
-// row (EPL a multiple of 4), CB components; lane sub ends with row sub.
-template <int L, int EPL, int CB>
+// FP64 sums (the FP64 form, and every field of several components: a mixed
+// operator's coefficients are widened, exactly): L lanes take L rows, each lane
+// EPL consecutive entries of every row (EPL a multiple of 4), CB components;
+// lane sub ends with row sub.
+template <int L, int EPL, int CB, class Coeff>
 __global__ void __launch_bounds__( 256 )
-    k_apply_pos64( int64_t n_tgt, int32_t const *__restrict__ pos, double const *__restrict__ coeff,
+    k_apply_pos64( int64_t n_tgt, int32_t const *__restrict__ pos, Coeff const *__restrict__ coeff,
                    double const *__restrict__ sorted, double *__restrict__ target, int64_t ps, int64_t cs_out,
                    uint32_t const *__restrict__ order )
 {
@@ -236,10 +265,9 @@ __global__ void __launch_bounds__( 256 )
         {
             int64_t const e = row * R + EPL * sub + q;
             int4 const ix = __ldcs( reinterpret_cast<int4 const *>( pos + e ) );
-            double2 const c0 = __ldcs( reinterpret_cast<double2 const *>( coeff + e ) );
-            double2 const c1 = __ldcs( reinterpret_cast<double2 const *>( coeff + e + 2 ) );
             int const at[4] = {ix.x, ix.y, ix.z, ix.w};
-            double const cj[4] = {c0.x, c0.y, c1.x, c1.y};
+            double cj[4];
+            load_coeff4( coeff + e, cj );
 #pragma unroll
             for ( int j = 0; j < 4; ++j )
             {
@@ -274,7 +302,7 @@ __global__ void __launch_bounds__( 256 )
 // sorted[CB p + k] = component c0 + k of source perm[p]
 template <int CB>
 __global__ void k_permute_fields( FieldView in, int64_t c0, uint32_t const *__restrict__ perm,
-                                  double *__restrict__ sorted64, float2 *__restrict__ sorted32 )
+                                  double *__restrict__ sorted )
 {
     int64_t const p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if ( p >= in.n )
@@ -282,44 +310,40 @@ __global__ void k_permute_fields( FieldView in, int64_t c0, uint32_t const *__re
     double const *v = in.base + ( perm ? (int64_t)__ldg( perm + p ) : p ) * in.ps + c0 * in.cs;
 #pragma unroll
     for ( int k = 0; k < CB; ++k )
-    {
-        double const x = __ldg( v + k * in.cs );
-        if ( sorted32 )
-        {
-            float const hi = __double2float_rn( x );
-            sorted32[CB * p + k] = make_float2( hi, __double2float_rn( x - (double)hi ) );
-        }
-        else
-            sorted64[CB * p + k] = x;
-    }
+        sorted[CB * p + k] = __ldg( v + k * in.cs );
 }
 
-// CB components of the rows; v64, v32: the values that pos points into.
-template <int CB>
-void launch_pos( int64_t n_rows, int R, int32_t const *pos, double const *coeff64, float const *coeff32,
-                 double const *v64, float2 const *v32, double *target, int64_t ps, int64_t cs, cudaStream_t s,
-                 uint32_t const *order )
+// fn( lanes a row, entries a lane ) of row length R
+template <class Fn>
+void for_row_shape( int R, Fn const &fn )
 {
-    auto const run = [&]( auto l, auto epl ) {
-        constexpr int L = decltype( l )::value, EPL = decltype( epl )::value;
-        if ( coeff32 )
-            k_apply_pos<L, EPL, CB><<<(unsigned)( ( n_rows * L + 255 ) / 256 ), 256, 0, s>>>(
-                n_rows, pos, coeff32, v32, target, ps, cs, order );
-        else
-            k_apply_pos64<L, EPL, CB><<<(unsigned)( ( n_rows + 255 ) / 256 ), 256, 0, s>>>(
-                n_rows, pos, coeff64, v64, target, ps, cs, order );
-        check_launch( "k_apply_pos" );
-    };
     std::integral_constant<int, 8> const eight;
     switch ( R )
     {
-    case 4: run( std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{} ); break;
-    case 8: run( std::integral_constant<int, 1>{}, eight ); break;
-    case 16: run( std::integral_constant<int, 2>{}, eight ); break;
-    case 32: run( std::integral_constant<int, 4>{}, eight ); break;
-    case 64: run( std::integral_constant<int, 8>{}, eight ); break;
-    default: run( std::integral_constant<int, 16>{}, eight ); break;
+    case 4: fn( std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{} ); break;
+    case 8: fn( std::integral_constant<int, 1>{}, eight ); break;
+    case 16: fn( std::integral_constant<int, 2>{}, eight ); break;
+    case 32: fn( std::integral_constant<int, 4>{}, eight ); break;
+    case 64: fn( std::integral_constant<int, 8>{}, eight ); break;
+    default: fn( std::integral_constant<int, 16>{}, eight ); break;
     }
+}
+
+// CB components of the rows, FP64 sums; values: what pos points into.
+template <int CB>
+void launch_pos64( int64_t n_rows, int R, int32_t const *pos, double const *coeff64, float const *coeff32,
+                   double const *values, double *target, int64_t ps, int64_t cs, cudaStream_t s,
+                   uint32_t const *order )
+{
+    for_row_shape( R, [&]( auto l, auto epl ) {
+        constexpr int L = decltype( l )::value, EPL = decltype( epl )::value;
+        unsigned const blocks = (unsigned)( ( n_rows + 255 ) / 256 );
+        if ( coeff32 )
+            k_apply_pos64<L, EPL, CB><<<blocks, 256, 0, s>>>( n_rows, pos, coeff32, values, target, ps, cs, order );
+        else
+            k_apply_pos64<L, EPL, CB><<<blocks, 256, 0, s>>>( n_rows, pos, coeff64, values, target, ps, cs, order );
+        check_launch( "k_apply_pos64" );
+    } );
 }
 
 } // namespace
@@ -349,9 +373,19 @@ SortedValues permute_values( int64_t n_src, uint32_t const *perm, double const *
 void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double const *coeff64, float const *coeff32,
                 SortedValues const &v, double *target, cudaStream_t s, uint32_t const *order )
 {
-    if ( n_rows > 0 )
-        launch_pos<1>( n_rows, uniform_row, pos, coeff64, coeff32, v.v64.get(), v.v32.get(), target, 1, 0, s,
-                       order );
+    if ( n_rows == 0 )
+        return;
+    if ( !coeff32 )
+    {
+        launch_pos64<1>( n_rows, uniform_row, pos, coeff64, nullptr, v.v64.get(), target, 1, 0, s, order );
+        return;
+    }
+    for_row_shape( uniform_row, [&]( auto l, auto epl ) {
+        constexpr int L = decltype( l )::value, EPL = decltype( epl )::value;
+        k_apply_pos<L, EPL><<<(unsigned)( ( n_rows * L + 255 ) / 256 ), 256, 0, s>>>( n_rows, pos, coeff32,
+                                                                                      v.v32.get(), target, order );
+        check_launch( "k_apply_pos" );
+    } );
 }
 
 void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
@@ -369,19 +403,14 @@ static void apply_fields( int64_t n_tgt, int uniform_row, int32_t const *pos, do
                           float const *coeff32, uint32_t const *perm, FieldView in, FieldView out, int64_t c0,
                           cudaStream_t s, uint32_t const *order )
 {
-    SortedValues v;
-    if ( coeff32 )
-        v.v32.allocate( std::max<int64_t>( 1, CB * in.n ), s );
-    else
-        v.v64.allocate( std::max<int64_t>( 1, CB * in.n ), s );
+    DeviceBuffer<double> v( std::max<int64_t>( 1, CB * in.n ), s );
     if ( in.n > 0 )
     {
-        k_permute_fields<CB><<<(unsigned)( ( in.n + 255 ) / 256 ), 256, 0, s>>>( in, c0, perm, v.v64.get(),
-                                                                                v.v32.get() );
+        k_permute_fields<CB><<<(unsigned)( ( in.n + 255 ) / 256 ), 256, 0, s>>>( in, c0, perm, v.get() );
         check_launch( "k_permute_fields" );
     }
-    launch_pos<CB>( n_tgt, uniform_row, pos, coeff64, coeff32, v.v64.get(), v.v32.get(), out.wbase + c0 * out.cs,
-                    out.ps, out.cs, s, order );
+    launch_pos64<CB>( n_tgt, uniform_row, pos, coeff64, coeff32, v.get(), out.wbase + c0 * out.cs, out.ps, out.cs, s,
+                      order );
 }
 
 void apply_sorted_multi( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
@@ -468,7 +497,7 @@ void apply_csr( int64_t n_tgt, int32_t const *offset, int32_t const *idx, double
     if ( !f32 && apply_sorted_supported( uniform_row ) )
     {
         // (a saved operator has no positions: the same sums by index)
-        launch_pos<1>( n_tgt, uniform_row, idx, coeff64, nullptr, values, nullptr, target, 1, 0, s, nullptr );
+        launch_pos64<1>( n_tgt, uniform_row, idx, coeff64, nullptr, values, target, 1, 0, s, nullptr );
         return;
     }
     int const len = uniform_row > 0 ? uniform_row : mean_row;
