@@ -31,6 +31,7 @@
 
 #include <algorithm>
 #include <new>
+#include <utility>
 
 namespace dtk
 {
@@ -650,24 +651,25 @@ void launch_adjoint_entries( dtk_mls_s const *h, AdjointView const &v, cudaStrea
     check_launch( "k_adjoint_entries" );
 }
 
+// (the handle takes the buffers once all of them are there: a call that runs
+// out of memory on the way can be made again)
 void build_transpose_for( dtk_mls_s *h, cudaStream_t s )
 {
     if ( h->t_offset.get() )
         return;
     int64_t const nnz = h->nnz, n_src = h->n_src;
     DeviceBuffer<uint32_t> keys( std::max<int64_t>( 1, nnz ), s );
-    h->t_entry.allocate( std::max<int64_t>( 1, nnz ), s );
+    DeviceBuffer<int32_t> t_entry( std::max<int64_t>( 1, nnz ), s ), t_offset( n_src + 1, s );
     unsigned const blocks = (unsigned)std::max<int64_t>( 1, ( nnz + 255 ) / 256 );
     if ( nnz )
     {
         k_entry_pairs<<<blocks, 256, 0, s>>>( h->idx.get(), nnz, keys.get(),
-                                              reinterpret_cast<uint32_t *>( h->t_entry.get() ) );
+                                              reinterpret_cast<uint32_t *>( t_entry.get() ) );
         check_launch( "k_entry_pairs" );
         int bits = 1;
         while ( ( int64_t( 1 ) << bits ) < n_src )
             ++bits;
-        radix_sort_pairs( keys.get(), reinterpret_cast<uint32_t *>( h->t_entry.get() ), nnz,
-                          ( bits + 7 ) / 8 * 8, s );
+        radix_sort_pairs( keys.get(), reinterpret_cast<uint32_t *>( t_entry.get() ), nnz, ( bits + 7 ) / 8 * 8, s );
     }
     DeviceBuffer<int64_t> counts( n_src, s ), offs( n_src + 1, s );
     DTK_CUDA_OR_THROW( cudaMemsetAsync( counts.get(), 0, n_src * sizeof( int64_t ), s ) );
@@ -677,16 +679,21 @@ void build_transpose_for( dtk_mls_s *h, cudaStream_t s )
         check_launch( "k_source_counts" );
     }
     exclusive_scan_i64( counts.get(), offs.get(), n_src, s );
-    h->t_offset.allocate( n_src + 1, s );
-    k_narrow<<<(unsigned)( ( n_src + 256 ) / 256 ), 256, 0, s>>>( offs.get(), h->t_offset.get(), n_src );
+    k_narrow<<<(unsigned)( ( n_src + 256 ) / 256 ), 256, 0, s>>>( offs.get(), t_offset.get(), n_src );
     check_launch( "k_narrow" );
-    if ( h->src_copy.get() && nnz )
-    {
-        // for the coordinate adjoint
-        h->t_place.allocate( nnz, s );
-        k_entry_places<<<blocks, 256, 0, s>>>( h->t_entry.get(), nnz, h->t_place.get() );
-        check_launch( "k_entry_places" );
-    }
+    h->t_entry = std::move( t_entry );
+    h->t_offset = std::move( t_offset );
+}
+
+// The entries' places in the transpose, for the coordinate adjoint.
+void build_places_for( dtk_mls_s *h, cudaStream_t s )
+{
+    if ( h->t_place.get() || h->nnz == 0 )
+        return;
+    DeviceBuffer<int32_t> t_place( h->nnz, s );
+    k_entry_places<<<(unsigned)( ( h->nnz + 255 ) / 256 ), 256, 0, s>>>( h->t_entry.get(), h->nnz, t_place.get() );
+    check_launch( "k_entry_places" );
+    h->t_place = std::move( t_place );
 }
 
 } // namespace
@@ -723,6 +730,7 @@ extern "C" dtk_status dtk_mls_apply_adjoint( dtk_mls_handle h, const double *cot
         DTK_CUDA_OR_THROW( cudaMemsetAsync( status.get(), 0, sizeof( unsigned ), s ) );
         if ( grad_coords && h->nnz )
         {
+            build_places_for( h, s );
             DeviceBuffer<double> contrib( 4 * h->nnz, s );
             AdjointView const v{h->src_copy.get(), h->tgt_copy.get(), h->offset.get(),  h->idx.get(),
                                 h->t_place.get(),  h->n_src,          h->opts.rbf,      source_values,

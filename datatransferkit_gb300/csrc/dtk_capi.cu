@@ -75,6 +75,7 @@ namespace
 {
 std::atomic<int64_t> g_jacobi_cap{0}, g_traversal_cap{0};
 std::atomic<int> g_jacobi_log{JACOBI_LOG};
+std::atomic<int64_t> g_failing_allocation{0};
 std::atomic<int> g_setup_lanes1{0}, g_setup_lanes2{0};
 }
 
@@ -87,6 +88,15 @@ unsigned long long jacobi_cap( int m )
 int jacobi_log_cap()
 {
     return g_jacobi_log.load( std::memory_order_relaxed );
+}
+
+void count_allocation()
+{
+    int64_t n = g_failing_allocation.load( std::memory_order_relaxed );
+    while ( n > 0 && !g_failing_allocation.compare_exchange_weak( n, n - 1, std::memory_order_relaxed ) )
+        ;
+    if ( n == 1 )
+        throw Error{DTK_ERR_OOM, "allocation refused (dtk_set_failing_allocation)"};
 }
 
 void fixed_setup_lanes( int &lanes1, int &lanes2 )
@@ -396,6 +406,14 @@ dtk_status dtk_set_rotation_log( int32_t rotations )
     return guarded( [&] {
         DTK_REQUIRE_OR_THROW( rotations >= 0 && rotations <= JACOBI_LOG, "rotations must be in [0, 160]" );
         g_jacobi_log.store( rotations, std::memory_order_relaxed );
+    } );
+}
+
+dtk_status dtk_set_failing_allocation( int64_t nth )
+{
+    return guarded( [&] {
+        DTK_REQUIRE_OR_THROW( nth >= 0, "nth must be >= 0" );
+        g_failing_allocation.store( nth, std::memory_order_relaxed );
     } );
 }
 

@@ -117,6 +117,9 @@ inline void validate_points( double const *p, int64_t n, int64_t ps, int64_t ds,
 // memory (the default pool returns them at every synchronization, and the
 // next create pays to map them again); dtk_release_cached_memory trims it.
 cudaMemPool_t device_pool();
+// Throws DTK_ERR_OOM in place of the allocation that
+// dtk_set_failing_allocation names.
+void count_allocation();
 
 // Stream-ordered device buffer from the library's pool (cudaFreeAsync frees).
 template <class T>
@@ -148,8 +151,10 @@ struct DeviceBuffer
         release();
         stream = s;
         n = count;
-        if ( count )
-            DTK_CUDA_OR_THROW( cudaMallocFromPoolAsync( (void **)&ptr, count * sizeof( T ), device_pool(), s ) );
+        if ( !count )
+            return;
+        count_allocation();
+        DTK_CUDA_OR_THROW( cudaMallocFromPoolAsync( (void **)&ptr, count * sizeof( T ), device_pool(), s ) );
     }
     void release()
     {

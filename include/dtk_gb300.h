@@ -420,6 +420,13 @@ dtk_status dtk_set_loop_caps(int64_t jacobi_rotations, int64_t traversal_steps);
  * [0, 160] -> DTK_ERR_INVALID_ARG. */
 dtk_status dtk_set_rotation_log(int32_t rotations);
 
+/* Lets the nth device allocation of this library from here on fail, for tests
+ * of what a call leaves behind that runs out of memory (no counterpart in the
+ * reference): that call returns DTK_ERR_OOM without asking the device, and the
+ * calls after it allocate as usual.  0: none (the default).  Negative values ->
+ * DTK_ERR_INVALID_ARG. */
+dtk_status dtk_set_failing_allocation(int64_t nth);
+
 /* Lanes a target in the gather phases of the persistent setup, for rows of
  * up to 32 entries and for longer rows (powers of two in [1, 32]; 0 = tuned
  * by timing, the default), for the batches created after it in this
