@@ -16,8 +16,8 @@
 //     neighbour (the last of largest rho in row order): the only term that
 //     needs the sum over the row, so one pass writes every entry's contribution
 //     and the farthest one is corrected after it.  The contributions cot_i
-//     dy/dx_j, with c_j cot_i beside them, are written at the entry's place in
-//     the transpose (one 32-byte sector each), so each source sums a run of
+//     dy/dx_j, with c_j beside them, are written at the entry's place in the
+//     transpose (one 32-byte sector each), so each source sums a run of
 //     consecutive sectors.  The pseudo-inverse is recomputed per target (never
 //     stored) from FP64 scaled moments.  Well-conditioned targets take an
 //     FP64 Cholesky (A^+ = A^-1 there); the rest take an FP32 round-robin
@@ -97,17 +97,19 @@ __global__ void k_transpose_gather( int64_t n_src, int32_t const *t_offset, int3
         int64_t const row = uniform_row > 0 ? e / uniform_row : row_of[e];
         double const c = F32 ? (double)static_cast<float const *>( coeff )[e]
                              : static_cast<double const *>( coeff )[e];
-        gv = __dadd_rn( gv, __dmul_rn( c, cot[row] ) );
+        gv = fma( c, cot[row], gv );
     }
     grad_values[s] = gv;
 }
 
-// The same sums and those of the coordinates from the entries' contributions,
-// which lie in the transpose's order (x, y, z, value: 32 bytes an entry): four
-// lanes a source, one a component, so that a warp reads whole lines.  1M x 1M,
-// k = 32: 1.47 ms as gathers through the entries' indices (three cache lines an
-// entry).
-__global__ void k_transpose_sum( int64_t n_src, int32_t const *t_offset, double const *contrib, double *grad_values,
+// The same sums, bit for bit, and those of the coordinates from the entries'
+// contributions, which lie in the transpose's order (x, y, z and the
+// coefficient: 32 bytes an entry): four lanes a source, one a component, so that
+// a warp reads whole lines; the lane of the values looks its entries' rows up.
+// 1M x 1M, k = 32: 1.47 ms as gathers through the entries' indices (three cache
+// lines an entry).
+__global__ void k_transpose_sum( int64_t n_src, int32_t const *t_offset, int32_t const *t_entry, int uniform_row,
+                                 int32_t const *row_of, double const *cot, double const *contrib, double *grad_values,
                                  double *grad_coords )
 {
     int64_t const t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -119,7 +121,15 @@ __global__ void k_transpose_sum( int64_t n_src, int32_t const *t_offset, double 
     double sum = 0.0;
 #pragma unroll 4
     for ( int64_t q = b; q < e; ++q )
-        sum = __dadd_rn( sum, __ldcs( contrib + 4 * q + c ) );
+    {
+        double by = 1.0;
+        if ( c == 3 )
+        {
+            unsigned const at = (unsigned)__ldcs( t_entry + q );
+            by = __ldg( cot + ( uniform_row > 0 ? (int)( at / (unsigned)uniform_row ) : row_of[at] ) );
+        }
+        sum = fma( __ldcs( contrib + 4 * q + c ), by, sum );
+    }
     if ( c == 3 )
         grad_values[s] = sum;
     else
@@ -138,16 +148,11 @@ struct AdjointView
     float const *coeff32;
     double *contrib; // 4 doubles an entry, in the transpose's order
     unsigned *status;
-    __device__ __forceinline__ void put( int64_t e, double x, double y, double z, double value ) const
+    __device__ __forceinline__ void put( int64_t e, double x, double y, double z ) const
     {
         double2 *const p = reinterpret_cast<double2 *>( contrib + 4 * (int64_t)place[e] );
         p[0] = make_double2( x, y );
-        p[1] = make_double2( z, value );
-    }
-    // the entry's part of grad_values
-    __device__ __forceinline__ double value( int64_t e, double ci ) const
-    {
-        return __dmul_rn( coeff32 ? (double)coeff32[e] : coeff64[e], ci );
+        p[1] = make_double2( z, coeff32 ? (double)coeff32[e] : coeff64[e] );
     }
 };
 
@@ -179,7 +184,7 @@ __device__ __forceinline__ bool adjoint_prologue( int64_t i, AdjointView const &
     if ( T.ci == 0.0 )
     {
         for ( int j = 0; j < T.len; ++j )
-            v.put( T.b0 + j, 0.0, 0.0, 0.0, v.value( T.b0 + j, T.ci ) );
+            v.put( T.b0 + j, 0.0, 0.0, 0.0 );
         return false;
     }
     T.tx = v.tgt[3 * i];
@@ -350,7 +355,7 @@ __device__ __forceinline__ void adjoint_passes( AdjTarget const &T, AdjointView 
         double const cx = scale * fma( gr, a.x, fma( pe, ga[0], -( pa * gz[0] ) ) ),
                      cy = scale * fma( gr, a.y, fma( pe, ga[1], -( pa * gz[1] ) ) ),
                      cz = scale * fma( gr, a.z, fma( pe, ga[2], -( pa * gz[2] ) ) );
-        v.put( T.b0 + j, cx, cy, cz, v.value( T.b0 + j, T.ci ) );
+        v.put( T.b0 + j, cx, cy, cz );
         if ( j == T.far )
         {
             fx = cx;
@@ -364,7 +369,7 @@ __device__ __forceinline__ void adjoint_passes( AdjTarget const &T, AdjointView 
     if ( T.radius_live )
     {
         double const r = -1.1 * S * scale;
-        v.put( T.b0 + T.far, fma( r, ux, fx ), fma( r, uy, fy ), fma( r, uz, fz ), v.value( T.b0 + T.far, T.ci ) );
+        v.put( T.b0 + T.far, fma( r, ux, fx ), fma( r, uy, fy ), fma( r, uz, fz ) );
     }
 }
 
@@ -728,6 +733,14 @@ extern "C" dtk_status dtk_mls_apply_adjoint( dtk_mls_handle h, const double *cot
         build_transpose_for( h, s );
         DeviceBuffer<unsigned> status( 1, s );
         DTK_CUDA_OR_THROW( cudaMemsetAsync( status.get(), 0, sizeof( unsigned ), s ) );
+        DeviceBuffer<int32_t> row_of;
+        if ( h->uniform_row <= 0 && h->nnz )
+        {
+            row_of.allocate( h->nnz, s );
+            k_entry_rows<<<(unsigned)( ( h->n_tgt + 255 ) / 256 ), 256, 0, s>>>( h->offset.get(), h->n_tgt,
+                                                                                 row_of.get() );
+            check_launch( "k_entry_rows" );
+        }
         if ( grad_coords && h->nnz )
         {
             build_places_for( h, s );
@@ -749,21 +762,14 @@ extern "C" dtk_status dtk_mls_apply_adjoint( dtk_mls_handle h, const double *cot
                 break;
             }
             k_transpose_sum<<<(unsigned)( ( 4 * h->n_src + 255 ) / 256 ), 256, 0, s>>>(
-                h->n_src, h->t_offset.get(), contrib.get(), grad_values, grad_coords );
+                h->n_src, h->t_offset.get(), h->t_entry.get(), h->uniform_row, row_of.get(), cot, contrib.get(),
+                grad_values, grad_coords );
             check_launch( "k_transpose_sum" );
         }
         else if ( h->n_src )
         {
             if ( grad_coords )
                 DTK_CUDA_OR_THROW( cudaMemsetAsync( grad_coords, 0, 3 * h->n_src * sizeof( double ), s ) );
-            DeviceBuffer<int32_t> row_of;
-            if ( h->uniform_row <= 0 && h->nnz )
-            {
-                row_of.allocate( h->nnz, s );
-                k_entry_rows<<<(unsigned)( ( h->n_tgt + 255 ) / 256 ), 256, 0, s>>>( h->offset.get(), h->n_tgt,
-                                                                                     row_of.get() );
-                check_launch( "k_entry_rows" );
-            }
             unsigned const blocks = (unsigned)( ( h->n_src + 255 ) / 256 );
             bool const f32 = h->coeff32.get() != nullptr;
             void const *coeff = f32 ? (void const *)h->coeff32.get() : (void const *)h->coeff64.get();
