@@ -59,3 +59,15 @@ def test_rows_of_a_radius():
     for coords in (False, True):
         gv, _ = op.apply_adjoint(dev(cot), dev(vals), coords=coords)
         assert np.array_equal(gv.cpu().numpy()[:12], want)
+
+
+@pytest.mark.parametrize("n_src", [704 * 700 + 1, 704 * 700 + 703])  # the larger blocks, a partial last one
+def test_many_sources(n_src):
+    src, tgt = syn.uniform_points(n_src, 85), syn.uniform_points(60000, 86)
+    cot = np.random.default_rng(5).standard_normal(len(tgt))
+    op = dtk.MovingLeastSquaresOperator(None, dev(src), dev(tgt), dtk.Wendland(2),
+                                        dtk.MultivariatePolynomialBasis(dtk.Linear, 3), k=8)
+    off, idx, coeff = (t.cpu().numpy() for t in op.csr())
+    some = [0, 703, 704, n_src - 1, *np.unique(idx)[:: 30000]]
+    gv, _ = op.apply_adjoint(dev(cot))
+    assert np.array_equal(gv.cpu().numpy()[some], fused_sums(off, idx, coeff, cot, some))
