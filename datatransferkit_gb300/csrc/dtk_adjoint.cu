@@ -197,20 +197,23 @@ __device__ __forceinline__ bool adjoint_prologue( int64_t i, AdjointView const &
     T.tx = v.tgt[3 * i];
     T.ty = v.tgt[3 * i + 1];
     T.tz = v.tgt[3 * i + 2];
-    // radius and the farthest neighbour (last of largest distance)
-    double d2max = 0.0;
-    T.far = 0;
-    for ( int j = 0; j < T.len; ++j )
-    {
+    auto const dist2 = [&]( int j ) {
         int64_t const sj = v.idx[T.b0 + j];
-        double const d2 = dist2_rn( v.src[3 * sj], v.src[3 * sj + 1], v.src[3 * sj + 2], T.tx, T.ty, T.tz );
-        if ( d2 >= d2max )
-        {
-            d2max = d2;
-            T.far = j;
-        }
-    }
+        return dist2_rn( v.src[3 * sj], v.src[3 * sj + 1], v.src[3 * sj + 2], T.tx, T.ty, T.tz );
+    };
+    double d2max = 0.0;
+    for ( int j = 0; j < T.len; ++j )
+        d2max = fmax( d2max, dist2( j ) );
     double const floor_d = 10. * DBL_EPSILON, dmax = sqrt( d2max );
+    // the farthest neighbour: the last of largest distance, which is not always
+    // one of largest square (two of them can have one root).  Looked for from
+    // the end, where a sorted row has it.
+    for ( T.far = T.len - 1; T.far > 0; --T.far )
+    {
+        double const d2 = dist2( T.far );
+        if ( d2 >= d2max || ( d2 >= d2max * ( 1.0 - 4.0 * DBL_EPSILON ) && sqrt( d2 ) >= dmax ) )
+            break;
+    }
     T.radius_live = dmax > floor_d;
     T.inv_r = 1.0 / ( 1.1 * ( T.radius_live ? dmax : floor_d ) );
     return true;
