@@ -220,7 +220,9 @@ __device__ __forceinline__ bool adjoint_prologue( int64_t i, AdjointView const &
 }
 
 // An entry's scaled coordinates, their squares, 1 / |x^| (0 at the target) and
-// |x^|: one reciprocal square root.
+// |x^|, from one reciprocal square root and a Newton step on the root's residual
+// (as accurate as a square root; without it, 2.6% faster at 1M x 1M, the 99th
+// percentile of the gradients' errors grew by 4% for Wendland<0>).
 struct AdjEntry
 {
     int64_t sj;
@@ -238,7 +240,8 @@ __device__ __forceinline__ AdjEntry adjoint_entry( AdjTarget const &T, AdjointVi
     a.zz = a.z * a.z;
     double const d2 = ( a.xx + a.yy ) + a.zz;
     a.inv_rho = d2 > 0.0 ? rsqrt( d2 ) : 0.0;
-    a.rho = d2 * a.inv_rho;
+    double const r = d2 * a.inv_rho;
+    a.rho = fma( fma( -r, r, d2 ), 0.5 * a.inv_rho, r );
     return a;
 }
 
