@@ -10,9 +10,9 @@
 // Rows of equal length R with R % 4 == 0 and R/4 a power of two (kNN rows,
 // e.g. R = 32) use R/8 lanes per row (8 entries each) with 128-bit loads:
 // int4 of indices and two double2 (FP64 form) or one float4 (mixed form) of
-// coefficients per 4 entries, then a shuffle reduction.  Other rows use S lanes
-// per row (S a power of two chosen from the mean row length) with coalesced
-// scalar loads.  Source values are
+// coefficients per 4 entries, then a shuffle reduction; a group of lanes may
+// take several rows.  Other rows use S lanes per row (S a power of two chosen
+// from the mean row length) with coalesced scalar loads.  Source values are
 // gathered through the read-only path; at 8M sources they are 64 MB and stay
 // resident in the 129 MB L2 while the CSR streams from HBM.
 #include "dtk_common.cuh"
@@ -85,27 +85,31 @@ bool is_pow2( int v ) { return v > 0 && ( v & ( v - 1 ) ) == 0; }
 } // namespace
 
 // ---------------------------------------------------------------------------
-// Apply over sorted positions (kNN operators): the source values are first
-// permuted into the tree's Morton order (one pass over the sources), and the
-// rows gather them by sorted position, so a row's neighbours sit in a few
-// sectors of an L2-resident array instead of 32 scattered ones.  The mixed
-// form keeps the permuted values as double-floats (hi = fl32(v), lo =
-// fl32(v - hi)) and sums c_j (hi_j + lo_j) in double-float arithmetic on the
-// FP32 pipe (TwoProd / TwoSum, the compensated scheme of the mixed setup):
-// the FP32 coefficients are the only rounding left, as with an FP64 sum.
-// The FP64 form permutes the doubles and sums with FP64 FMAs, whose pipe bounds
-// it (64 cycles an instruction a warp): one FMA an entry, and the lanes' partial
-// sums of a row are added for as many rows as there are lanes at once, each
-// lane ending with one row (2M rows of 32 with the permutation 257 -> 201 us,
-// 118 us of them the bytes).  A field of several components keeps a point's
-// components side by side, up to four a pass, so that positions and
-// coefficients are read once.  Its sums are FP64 in both forms (a double-float
-// has FP32's range and 48 bits); FP32 coefficients are widened on the integer
-// pipe.  Three components of 1M rows of 32, mixed: 480 us by index, 202 us so,
-// 269 with the conversions on the FP64 pipe.  Rows go in
-// the targets' Morton order when the operator has it, so that consecutive
-// rows share most of their neighbours' values in L1 (0.70 -> 0.59 ms for 8M
-// rows of 32; 16 entries a lane instead of 8 was 1.26 ms, 4 no different).
+// Apply over uniform rows.
+//
+// Mixed form, one component: the source values are first permuted into the
+// tree's Morton order (one pass over the sources) as double-floats (hi =
+// fl32(v), lo = fl32(v - hi)), and the rows gather them by sorted position, so a
+// row's neighbours sit in a few sectors of an L2-resident array instead of 32
+// scattered ones; c_j (hi_j + lo_j) is summed in double-float arithmetic on the
+// FP32 pipe (TwoProd / TwoSum, the compensated scheme of the mixed setup): the
+// FP32 coefficients are the only rounding left, as with an FP64 sum, for values
+// in FP32's range.
+//
+// FP64 sums, for the FP64 form and for fields of several components in both (a
+// double-float has FP32's range and 48 bits): FP64 FMAs, whose pipe bounds them
+// with the bytes (64 cycles an instruction a warp), by index from the field as
+// it is, up to four components a thread, so that indices and coefficients are
+// read once; FP32 coefficients are widened on the integer pipe.  Large fields of
+// several components go through a sorted copy, a point's components side by
+// side.  FP64 form, 2M rows of 32: 257 us by sorted position with a reduction
+// a row of 4 entries a lane, 169 us so (118 us are the bytes); three components
+// of 1M rows, mixed: 480 us with 8 lanes a row and scalar loads, 187 us so (269
+// with the conversions on the FP64 pipe).
+//
+// Rows go in the targets' Morton order when the operator has it, so that
+// consecutive rows share most of their neighbours' values in L1 (0.70 -> 0.59 ms
+// for 8M rows of 32; 16 entries a lane instead of 8 was 1.26 ms, 4 no different).
 // ---------------------------------------------------------------------------
 namespace
 {
@@ -236,92 +240,127 @@ __global__ void __launch_bounds__( 256 )
         target[row] = sum;
 }
 
-// FP64 sums (the FP64 form, and every field of several components: a mixed
-// operator's coefficients are widened, exactly): L lanes take L rows, each lane
-// EPL consecutive entries of every row (EPL a multiple of 4), CB components;
-// lane sub ends with row sub.
-template <int L, int EPL, int CB, class Coeff>
-__global__ void __launch_bounds__( 256 )
-    k_apply_pos64( int64_t n_tgt, int32_t const *__restrict__ pos, Coeff const *__restrict__ coeff,
-                   double const *__restrict__ sorted, double *__restrict__ target, int64_t ps, int64_t cs_out,
-                   uint32_t const *__restrict__ order )
+// FP64 sums of CB components from c0 on: L lanes take ROWS rows, each lane EPL
+// consecutive entries of every row (EPL a multiple of 4).  mine: the row that
+// this lane ends with, -1 for none.  PACKED: the field has CB components side by
+// side.
+template <int L, int EPL, int ROWS, int CB, bool PACKED, class Coeff>
+__device__ __forceinline__ void rows64( int32_t const *__restrict__ at, Coeff const *__restrict__ coeff,
+                                        FieldView const &in, FieldView const &out, int64_t c0, int64_t mine )
 {
-    constexpr int R = EPL * L;
-    int64_t const at0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; // this lane's row in order
+    constexpr int R = EPL * L, SHARE = L / ROWS; // lanes that end with the same row
     int const sub = threadIdx.x % L;
-    int64_t const mine = at0 < n_tgt ? ( order ? (int64_t)__ldg( order + at0 ) : at0 ) : -1;
-    double a[L][CB];
+    double a[ROWS][CB];
 #pragma unroll
-    for ( int r = 0; r < L; ++r )
+    for ( int r = 0; r < ROWS; ++r )
     {
 #pragma unroll
         for ( int k = 0; k < CB; ++k )
             a[r][k] = 0.0;
-        int64_t const row = L > 1 ? __shfl_sync( FULL, mine, r, L ) : mine;
+        int64_t const row = L > 1 ? __shfl_sync( FULL, mine, r * SHARE, L ) : mine;
         if ( row < 0 )
             continue;
 #pragma unroll
         for ( int q = 0; q < EPL; q += 4 )
         {
             int64_t const e = row * R + EPL * sub + q;
-            int4 const ix = __ldcs( reinterpret_cast<int4 const *>( pos + e ) );
-            int const at[4] = {ix.x, ix.y, ix.z, ix.w};
+            int4 const ix = __ldcs( reinterpret_cast<int4 const *>( at + e ) );
+            int const p[4] = {ix.x, ix.y, ix.z, ix.w};
             double cj[4];
             load_coeff4( coeff + e, cj );
 #pragma unroll
             for ( int j = 0; j < 4; ++j )
             {
-                double const *v = sorted + (int64_t)CB * at[j];
+                double const *v = PACKED ? in.base + (int64_t)CB * p[j] : in.base + p[j] * in.ps + c0 * in.cs;
 #pragma unroll
                 for ( int k = 0; k < CB; ++k )
-                    a[r][k] = fma( cj[j], __ldg( v + k ), a[r][k] );
+                    a[r][k] = fma( cj[j], __ldg( v + ( PACKED ? k : k * in.cs ) ), a[r][k] );
             }
         }
     }
-    // halve the rows a lane holds until one is left
+    // halve the rows a lane holds until one is left, then add up its lanes
 #pragma unroll
-    for ( int o = L / 2; o > 0; o >>= 1 )
+    for ( int n = ROWS / 2, o = L / 2; n > 0; n >>= 1, o >>= 1 )
     {
         bool const upper = ( sub & o ) != 0;
 #pragma unroll
-        for ( int r = 0; r < o; ++r )
+        for ( int r = 0; r < n; ++r )
 #pragma unroll
             for ( int k = 0; k < CB; ++k )
             {
-                double const give = upper ? a[r][k] : a[r + o][k];
-                double const keep = upper ? a[r + o][k] : a[r][k];
+                double const give = upper ? a[r][k] : a[r + n][k];
+                double const keep = upper ? a[r + n][k] : a[r][k];
                 a[r][k] = keep + __shfl_xor_sync( FULL, give, o );
             }
     }
-    if ( mine >= 0 )
+#pragma unroll
+    for ( int o = SHARE / 2; o > 0; o >>= 1 )
 #pragma unroll
         for ( int k = 0; k < CB; ++k )
-            target[mine * ps + k * cs_out] = a[0][k];
+            a[0][k] += __shfl_xor_sync( FULL, a[0][k], o );
+    if ( mine >= 0 && sub % SHARE == 0 )
+#pragma unroll
+        for ( int k = 0; k < CB; ++k )
+            out.wbase[mine * out.ps + ( c0 + k ) * out.cs] = a[0][k];
 }
 
-// sorted[CB p + k] = component c0 + k of source perm[p]
-template <int CB>
-__global__ void k_permute_fields( FieldView in, int64_t c0, uint32_t const *__restrict__ perm,
+// FP64 sums (the FP64 form, and every field of several components: a mixed
+// operator's coefficients are widened, exactly) of n_full groups of CB
+// components and others of CB - 1 behind them, in one launch (a component that
+// is only masked out takes the FP64 pipe as long as a real one).  `at` indexes
+// the values: a sorted copy of the field or the field itself.  A row's partial
+// sums meet in the same order whatever ROWS is and wherever the values lie, so
+// every path gives the same bits.
+template <int L, int EPL, int ROWS, int CB, bool PACKED, class Coeff>
+__global__ void __launch_bounds__( 256 )
+    k_apply_rows64( int64_t n_rows, int32_t const *__restrict__ at, Coeff const *__restrict__ coeff, FieldView in,
+                    FieldView out, int64_t n_full, uint32_t const *__restrict__ order )
+{
+    static_assert( ROWS <= L && L % ROWS == 0, "a lane ends with one row at most" );
+    int64_t const gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    int64_t const first = gt / L * ROWS + threadIdx.x % L / ( L / ROWS ); // this lane's row in order
+    int64_t const mine = first < n_rows ? ( order ? (int64_t)__ldg( order + first ) : first ) : -1;
+    if constexpr ( PACKED )
+    {
+        rows64<L, EPL, ROWS, CB, true>( at, coeff, in, out, 0, mine );
+        return;
+    }
+    for ( int64_t g = blockIdx.y;; g += gridDim.y )
+    {
+        int64_t const c0 = g < n_full ? g * CB : g * CB - ( g - n_full );
+        if ( c0 >= in.n_comp )
+            break;
+        if ( g < n_full )
+            rows64<L, EPL, ROWS, CB, false>( at, coeff, in, out, c0, mine );
+        else if constexpr ( CB > 1 )
+            rows64<L, EPL, ROWS, CB - 1, false>( at, coeff, in, out, c0, mine );
+    }
+}
+
+// sorted[nc p + k] = component c0 + k < c0 + nc of source perm[p]
+__global__ void k_permute_fields( FieldView in, int64_t c0, int nc, uint32_t const *__restrict__ perm,
                                   double *__restrict__ sorted )
 {
     int64_t const p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if ( p >= in.n )
         return;
-    double const *v = in.base + ( perm ? (int64_t)__ldg( perm + p ) : p ) * in.ps + c0 * in.cs;
+    double const *v = in.base + (int64_t)__ldg( perm + p ) * in.ps + c0 * in.cs;
 #pragma unroll
-    for ( int k = 0; k < CB; ++k )
-        sorted[CB * p + k] = __ldg( v + k * in.cs );
+    for ( int k = 0; k < 4; ++k )
+        if ( k < nc )
+            sorted[nc * p + k] = __ldg( v + k * in.cs );
 }
 
-// fn( lanes a row, entries a lane ) of row length R
-template <class Fn>
+// fn( lanes a row, entries a lane ) of row length R, with SHORTEST entries a
+// lane for rows of 8
+template <int SHORTEST, class Fn>
 void for_row_shape( int R, Fn const &fn )
 {
     std::integral_constant<int, 8> const eight;
     switch ( R )
     {
     case 4: fn( std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{} ); break;
-    case 8: fn( std::integral_constant<int, 1>{}, eight ); break;
+    case 8: fn( std::integral_constant<int, 8 / SHORTEST>{}, std::integral_constant<int, SHORTEST>{} ); break;
     case 16: fn( std::integral_constant<int, 2>{}, eight ); break;
     case 32: fn( std::integral_constant<int, 4>{}, eight ); break;
     case 64: fn( std::integral_constant<int, 8>{}, eight ); break;
@@ -329,21 +368,66 @@ void for_row_shape( int R, Fn const &fn )
     }
 }
 
-// CB components of the rows, FP64 sums; values: what pos points into.
-template <int CB>
-void launch_pos64( int64_t n_rows, int R, int32_t const *pos, double const *coeff64, float const *coeff32,
-                   double const *values, double *target, int64_t ps, int64_t cs, cudaStream_t s,
-                   uint32_t const *order )
+// FP64 sums of every component in one launch, up to four components a thread.
+// A group of lanes takes one row where the adds over its lanes are cheap beside
+// the latency (up to two components, or few rows), otherwise up to four rows
+// (us, one row / four: 2M rows of 32, FP64 form, 1 component 169 / 239, 2
+// components 301 / 325, on a sorted copy 314 / 281; 3 components 423 / 406, mixed
+// 421 / 368; 10k rows, 3 components 10.9 / 12.4).
+template <int CB, class Coeff>
+void launch_rows64( int64_t n_rows, int R, int32_t const *at, Coeff const *coeff, FieldView const &in,
+                    FieldView const &out, int64_t groups, bool sorted, cudaStream_t s, uint32_t const *order )
 {
-    for_row_shape( R, [&]( auto l, auto epl ) {
+    int64_t const n_full = in.n_comp - groups * ( CB - 1 );
+    bool const packed = in.n_comp == CB && in.ps == CB && ( CB == 1 || in.cs == 1 );
+    bool const several = n_rows >= 100000 && ( CB >= 3 || ( CB == 2 && sorted ) );
+    for_row_shape<4>( R, [&]( auto l, auto epl ) {
         constexpr int L = decltype( l )::value, EPL = decltype( epl )::value;
-        unsigned const blocks = (unsigned)( ( n_rows + 255 ) / 256 );
-        if ( coeff32 )
-            k_apply_pos64<L, EPL, CB><<<blocks, 256, 0, s>>>( n_rows, pos, coeff32, values, target, ps, cs, order );
+        constexpr int MOST = CB == 1 || L == 1 ? 1 : L < 4 ? L : 4;
+        auto const run = [&]( auto rows, auto is_packed ) {
+            constexpr int ROWS = decltype( rows )::value;
+            dim3 const grid( (unsigned)( ( ( n_rows + ROWS - 1 ) / ROWS * L + 255 ) / 256 ),
+                             (unsigned)std::min<int64_t>( groups, 65535 ) );
+            k_apply_rows64<L, EPL, ROWS, CB, decltype( is_packed )::value>
+                <<<grid, 256, 0, s>>>( n_rows, at, coeff, in, out, n_full, order );
+            check_launch( "k_apply_rows64" );
+        };
+        auto const run_rows = [&]( auto rows ) {
+            if ( packed )
+                run( rows, std::true_type{} );
+            else
+                run( rows, std::false_type{} );
+        };
+        if ( several )
+            run_rows( std::integral_constant<int, MOST>{} );
         else
-            k_apply_pos64<L, EPL, CB><<<blocks, 256, 0, s>>>( n_rows, pos, coeff64, values, target, ps, cs, order );
-        check_launch( "k_apply_pos64" );
+            run_rows( std::integral_constant<int, 1>{} );
     } );
+}
+
+void apply_rows64( int64_t n_rows, int R, int32_t const *at, double const *coeff64, float const *coeff32,
+                   FieldView const &in, FieldView const &out, bool sorted, cudaStream_t s, uint32_t const *order )
+{
+    int64_t const groups = ( in.n_comp + 3 ) / 4, cb = ( in.n_comp + groups - 1 ) / groups;
+    auto const run = [&]( auto c ) {
+        constexpr int CB = decltype( c )::value;
+        if ( coeff32 )
+            launch_rows64<CB>( n_rows, R, at, coeff32, in, out, groups, sorted, s, order );
+        else
+            launch_rows64<CB>( n_rows, R, at, coeff64, in, out, groups, sorted, s, order );
+    };
+    switch ( cb )
+    {
+    case 1: run( std::integral_constant<int, 1>{} ); break;
+    case 2: run( std::integral_constant<int, 2>{} ); break;
+    case 3: run( std::integral_constant<int, 3>{} ); break;
+    default: run( std::integral_constant<int, 4>{} ); break;
+    }
+}
+
+FieldView rank1( double const *values, double *target, int64_t n )
+{
+    return FieldView{values, target, n, 1, 1, 0};
 }
 
 } // namespace
@@ -377,10 +461,11 @@ void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double cons
         return;
     if ( !coeff32 )
     {
-        launch_pos64<1>( n_rows, uniform_row, pos, coeff64, nullptr, v.v64.get(), target, 1, 0, s, order );
+        apply_rows64( n_rows, uniform_row, pos, coeff64, nullptr, rank1( v.v64.get(), nullptr, 0 ),
+                      rank1( nullptr, target, n_rows ), true, s, order );
         return;
     }
-    for_row_shape( uniform_row, [&]( auto l, auto epl ) {
+    for_row_shape<8>( uniform_row, [&]( auto l, auto epl ) {
         constexpr int L = decltype( l )::value, EPL = decltype( epl )::value;
         k_apply_pos<L, EPL><<<(unsigned)( ( n_rows * L + 255 ) / 256 ), 256, 0, s>>>( n_rows, pos, coeff32,
                                                                                       v.v32.get(), target, order );
@@ -388,44 +473,48 @@ void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double cons
     } );
 }
 
-void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
+void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *idx, int32_t const *pos, double const *coeff64,
                    float const *coeff32, int64_t n_src, uint32_t const *perm, double const *values,
                    double *target, cudaStream_t s, uint32_t const *order )
 {
     if ( n_tgt == 0 )
         return;
-    SortedValues const v = permute_values( n_src, perm, values, coeff32 != nullptr, s );
-    apply_pos( n_tgt, uniform_row, pos, coeff64, coeff32, v, target, s, order );
-}
-
-template <int CB>
-static void apply_fields( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
-                          float const *coeff32, uint32_t const *perm, FieldView in, FieldView out, int64_t c0,
-                          cudaStream_t s, uint32_t const *order )
-{
-    DeviceBuffer<double> v( std::max<int64_t>( 1, CB * in.n ), s );
-    if ( in.n > 0 )
+    if ( coeff64 )
     {
-        k_permute_fields<CB><<<(unsigned)( ( in.n + 255 ) / 256 ), 256, 0, s>>>( in, c0, perm, v.get() );
-        check_launch( "k_permute_fields" );
+        apply_rows64( n_tgt, uniform_row, idx, coeff64, nullptr, rank1( values, nullptr, n_src ),
+                      rank1( nullptr, target, n_tgt ), false, s, order );
+        return;
     }
-    launch_pos64<CB>( n_tgt, uniform_row, pos, coeff64, coeff32, v.get(), out.wbase + c0 * out.cs, out.ps, out.cs, s,
-                      order );
+    SortedValues const v = permute_values( n_src, pos ? perm : nullptr, values, true, s );
+    apply_pos( n_tgt, uniform_row, pos ? pos : idx, nullptr, coeff32, v, target, s, order );
 }
 
-void apply_sorted_multi( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
-                         float const *coeff32, uint32_t const *perm, FieldView in, FieldView out, cudaStream_t s,
-                         uint32_t const *order )
+void apply_sorted_multi( int64_t n_tgt, int uniform_row, int32_t const *idx, int32_t const *pos,
+                         double const *coeff64, float const *coeff32, uint32_t const *perm, FieldView in,
+                         FieldView out, cudaStream_t s, uint32_t const *order )
 {
     if ( n_tgt == 0 )
         return;
-    for ( int64_t c0 = 0; c0 < in.n_comp; c0 += 4 )
+    // A sorted copy pays from about 2M sources on, when the fields outgrow the
+    // caches of L2's nearer half, with at least 16 entries a source (us, by
+    // index / on a copy, as many targets: 2M, rows of 16, 3 components 274 / 261;
+    // 4M, rows of 16, 2 components 539 / 466, 3 components 734 / 580, rows of 32
+    // 882 / 789; but 1M, rows of 32, 3 components 202 / 206; 4M to 1M, rows of 32
+    // 261 / 273; 4M to 30k 15 / 81)
+    if ( !( pos && in.n_comp > 1 && in.n >= 2000000 && n_tgt * uniform_row >= 16 * in.n ) )
     {
-        auto const run = in.n_comp - c0 >= 4   ? apply_fields<4>
-                         : in.n_comp - c0 == 3 ? apply_fields<3>
-                         : in.n_comp - c0 == 2 ? apply_fields<2>
-                                               : apply_fields<1>;
-        run( n_tgt, uniform_row, pos, coeff64, coeff32, perm, in, out, c0, s, order );
+        apply_rows64( n_tgt, uniform_row, idx, coeff64, coeff32, in, out, false, s, order );
+        return;
+    }
+    int64_t const groups = ( in.n_comp + 3 ) / 4, cb = ( in.n_comp + groups - 1 ) / groups;
+    DeviceBuffer<double> v( cb * in.n, s );
+    for ( int64_t c0 = 0; c0 < in.n_comp; c0 += cb )
+    {
+        int64_t const nc = std::min( cb, in.n_comp - c0 );
+        k_permute_fields<<<(unsigned)( ( in.n + 255 ) / 256 ), 256, 0, s>>>( in, c0, (int)nc, perm, v.get() );
+        check_launch( "k_permute_fields" );
+        apply_rows64( n_tgt, uniform_row, pos, coeff64, coeff32, FieldView{v.get(), nullptr, in.n, nc, nc, 1},
+                      FieldView{nullptr, out.wbase + c0 * out.cs, n_tgt, nc, out.ps, out.cs}, true, s, order );
     }
 }
 
@@ -497,7 +586,8 @@ void apply_csr( int64_t n_tgt, int32_t const *offset, int32_t const *idx, double
     if ( !f32 && apply_sorted_supported( uniform_row ) )
     {
         // (a saved operator has no positions: the same sums by index)
-        launch_pos64<1>( n_tgt, uniform_row, idx, coeff64, nullptr, values, target, 1, 0, s, nullptr );
+        apply_rows64( n_tgt, uniform_row, idx, coeff64, nullptr, rank1( values, nullptr, 0 ),
+                      rank1( nullptr, target, n_tgt ), false, s, nullptr );
         return;
     }
     int const len = uniform_row > 0 ? uniform_row : mean_row;

@@ -584,13 +584,10 @@ dtk_status dtk_mls_apply( dtk_mls_handle h, const double *source_values, int64_t
         require_device_memory( target_values, "target_values" );
         cudaStream_t s = reinterpret_cast<cudaStream_t>( stream_ );
         TouchOnExit const touch{&h->life, s};
-        // uniform rows: by sorted position when the search left them; the
-        // mixed form always (its double-float sum), by index otherwise
-        bool const by_pos = h->pos.get() && h->perm.get();
-        if ( apply_sorted_supported( h->uniform_row ) && ( by_pos || h->coeff32.get() ) )
-            apply_sorted( h->n_tgt, h->uniform_row, by_pos ? h->pos.get() : h->idx.get(), h->coeff64.get(),
-                          h->coeff32.get(), h->n_src, by_pos ? h->perm.get() : nullptr, source_values,
-                          target_values, s, by_pos ? h->order.get() : nullptr );
+        if ( apply_sorted_supported( h->uniform_row ) )
+            apply_sorted( h->n_tgt, h->uniform_row, h->idx.get(), h->perm.get() ? h->pos.get() : nullptr,
+                          h->coeff64.get(), h->coeff32.get(), h->n_src, h->perm.get(), source_values, target_values,
+                          s, h->order.get() );
         else
             apply_csr( h->n_tgt, h->offset.get(), h->idx.get(), h->coeff64.get(), h->coeff32.get(),
                        h->uniform_row, h->mean_row, source_values, target_values, s );

@@ -718,13 +718,16 @@ SortedValues permute_values( int64_t n_src, uint32_t const *perm, double const *
 // share most of their neighbours' values in L1) or in row order
 void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double const *coeff64, float const *coeff32,
                 SortedValues const &v, double *target, cudaStream_t s, uint32_t const *order = nullptr );
-// several components, up to four a pass
-void apply_sorted_multi( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
-                         float const *coeff32, uint32_t const *perm, FieldView in, FieldView out, cudaStream_t s,
-                         uint32_t const *order );
-void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *pos, double const *coeff64,
+// A whole operator with uniform rows, by index (idx) or, where pos is not null
+// and it pays, by sorted position on a copy of the values; the FP64 sums are the
+// same bits either way.  A mixed operator's rank-1 field is summed in
+// double-float (always on a copy), its fields of several components in FP64.
+void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *idx, int32_t const *pos, double const *coeff64,
                    float const *coeff32, int64_t n_src, uint32_t const *perm, double const *values,
-                   double *target, cudaStream_t s, uint32_t const *order = nullptr );
+                   double *target, cudaStream_t s, uint32_t const *order );
+void apply_sorted_multi( int64_t n_tgt, int uniform_row, int32_t const *idx, int32_t const *pos,
+                         double const *coeff64, float const *coeff32, uint32_t const *perm, FieldView in,
+                         FieldView out, cudaStream_t s, uint32_t const *order );
 
 // Adjoint kernels.
 struct AdjointArgs

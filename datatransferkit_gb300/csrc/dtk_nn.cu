@@ -184,13 +184,9 @@ dtk_status dtk_mls_apply_multi( dtk_mls_handle h, const double *source_values, i
         out.wbase = target_values;
         cudaStream_t s = reinterpret_cast<cudaStream_t>( stream_ );
         TouchOnExit const touch{&h->life, s};
-        // uniform rows as the rank-1 apply takes them: by sorted position, the
-        // mixed form by index otherwise
-        bool const by_pos = h->pos.get() && h->perm.get();
-        if ( apply_sorted_supported( h->uniform_row ) && ( by_pos || h->coeff32.get() ) )
-            apply_sorted_multi( h->n_tgt, h->uniform_row, by_pos ? h->pos.get() : h->idx.get(), h->coeff64.get(),
-                                h->coeff32.get(), by_pos ? h->perm.get() : nullptr, in, out, s,
-                                by_pos ? h->order.get() : nullptr );
+        if ( apply_sorted_supported( h->uniform_row ) )
+            apply_sorted_multi( h->n_tgt, h->uniform_row, h->idx.get(), h->perm.get() ? h->pos.get() : nullptr,
+                                h->coeff64.get(), h->coeff32.get(), h->perm.get(), in, out, s, h->order.get() );
         else
             apply_csr_multi( h->n_tgt, h->offset.get(), h->idx.get(), h->coeff64.get(), h->coeff32.get(), in,
                              out, s );
