@@ -494,6 +494,57 @@ __host__ __device__ __forceinline__ bool fx_load( State const &st, bool live )
     return st.both( ok );
 }
 
+constexpr int FX_TRUNCATE = -51; // twice DBL_EPSILON's exponent less one
+
+// Pivots K .. of the LDL^T of a, in units of 2^(d_i + d_j).
+template <int M, int K, class State>
+__host__ __device__ __forceinline__ void fx_pivots( State const &st, float ( &a )[M][M], bool &truncates )
+{
+    // (no pivot is taken for smaller than its rounding, 2^-17)
+    float const d = a[K][K] > 7.6293945e-6f ? a[K][K] : 7.6293945e-6f;
+    // d 2^(2 d_K) < 2^FX_TRUNCATE, with a margin for the FP32 sums
+    truncates |= d * 1.125f < fx_pow2( FX_TRUNCATE - 2 * st.exp( K ) );
+    if constexpr ( K + 1 < M )
+    {
+        float const r = 1.0f / d;
+#pragma unroll
+        for ( int i = K + 1; i < M; ++i )
+        {
+            float const l = a[K][i] * r;
+#pragma unroll
+            for ( int j = K + 1; j < M; ++j )
+                if ( j >= i )
+                    a[i][j] = fx_fma( -l, a[K][j], a[i][j] );
+        }
+        fx_pivots<M, K + 1>( st, a, truncates );
+    }
+}
+
+// The smallest eigenvalue is at most the truncation threshold, so that the
+// matrix would be handed back at the end: one of the pivots of an LDL^T of F in
+// FP32 is (each bounds it from above, as the smallest eigenvalue of a leading
+// block does).  Without it clouds of so small a scale paid for both forms: 300k
+// quadratic targets in a cube of edge 0.01 took 9.8 ms, now 8.6 (FP64 alone
+// 7.4); at edge 1, where no matrix is handed back, it costs 0.04 of 8.25 ms.
+template <int M, class State>
+__host__ __device__ __forceinline__ bool fx_truncates( State const &st )
+{
+    using Lay = FxLayout<M>;
+    float a[M][M]; // the upper triangle, in units of 2^(d_i + d_j)
+    bool truncates = false;
+#pragma unroll
+    for ( int i = 0; i < M; ++i )
+    {
+        a[i][i] = (float)(int32_t)( st.diag( i ) >> 30 ) * 9.3132257e-10f; // 2^-30
+#pragma unroll
+        for ( int j = 1; j < M; ++j )
+            if ( j > i )
+                a[i][j] = fx_float( st.f( Lay::pair( i, j ) ) ) * 1.6155871e-27f; // 2^-89
+    }
+    fx_pivots<M, 0>( st, a, truncates );
+    return truncates;
+}
+
 // The slot of the largest |E(i, j)|, first in row-major order, compared
 // exactly.
 template <int M, class State>
@@ -567,6 +618,7 @@ template <int M, class State>
 __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, bool live )
 {
     using Lay = FxLayout<M>;
+    live = live && !fx_truncates<M>( st );
     int const d0 = live ? st.exp( 0 ) : 0; // V's unit
     int fv = FX_V;                         // 2^fv is 1 in it
     int it = 0;
@@ -724,7 +776,7 @@ __host__ __device__ __forceinline__ int fx_jacobi( State const &st, int cap, boo
             int64_t const f = st.diag( k );
             FxNum<2> const v = st.v( k );
             // E(k, k) at least twice the truncation threshold
-            ok = f > 0 && 63 - fx_clz( (uint64_t)f ) + 2 * d - FX_ONE >= -51;
+            ok = f > 0 && 63 - fx_clz( (uint64_t)f ) + 2 * d - FX_ONE >= FX_TRUNCATE;
             double w = 0.0;
             if ( ok && !fx_zero( v ) )
             {

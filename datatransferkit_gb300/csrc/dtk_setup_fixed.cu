@@ -47,6 +47,18 @@ __device__ __forceinline__ Support support_of( double d2max )
     return Support{radius, 1.0 / radius};
 }
 
+// A diagonal moment, and with it the smallest eigenvalue, is certainly below the
+// truncation threshold: the least over the axes of the sum of phi x^2 (M = 4;
+// phi x^2 y^2, M = 10) is at most 1/3 (1/9) of that of phi rho^2 (rho^4), and
+// phi(q) q^2 1.1^2 / 3 < 0.125, phi(q) q^4 1.1^4 / 9 < 0.0125 for every positive
+// phi.  Such a row is the FP64 kernel's, before its moments are summed.
+template <int M>
+__device__ __forceinline__ bool truncates_by_size( double d2max, int len )
+{
+    double const most = M == 10 ? 0.0125 * ( d2max * d2max ) : 0.125 * d2max;
+    return M > 1 && len * most < 4.440892098500626e-16; // 2^FX_TRUNCATE
+}
+
 // phi of a neighbour, rounded as the reference rounds it: ill-conditioned rows
 // carry an ulp of a weight into the twelfth digit of their coefficients.  The
 // quotient |x| / radius comes from the reciprocal and one residual (3 FP64
@@ -408,6 +420,8 @@ __device__ __forceinline__ unsigned fixed_targets( Neighbours const &nb, PointsV
         for ( int o = rows_sorted ? 0 : G >> 1; o; o >>= 1 )
             d2max = fmax( d2max, __shfl_xor_sync( FULL, d2max, o ) );
         Support const sup = support_of( d2max );
+        if ( truncates_by_size<M>( d2max, len ) )
+            len = 0; // (no moments: handed back)
         double A[N_MOMENTS<M>];
 #pragma unroll
         for ( int u = 0; u < N_MOMENTS<M>; ++u )
