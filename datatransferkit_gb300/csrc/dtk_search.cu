@@ -1075,8 +1075,8 @@ constexpr float LIST_GROWTH = 1.5f;
 // seeds the next): n_big chunks of seq queries, then chunks of seq / 2 up to
 // the end, so that the warps finish close together.  A warp takes the next
 // chunk from a counter as soon as it is done with one.
-// Of a list (n_listed, its length on the device) the chunks are as long as
-// leaves four to every warp of the launch, and seq at most.
+// Of a list (n_listed, its length on the device: 0 and the launch is empty) the
+// chunks are as long as leaves four to every warp of the launch, and seq at most.
 struct KnnChunks
 {
     int seq;
@@ -1218,8 +1218,9 @@ __global__ void __launch_bounds__( Q_WARPS * 32, KNN_BLOCKS_PER_SM )
     int64_t const n_queries = ch.n_listed ? (int64_t)*ch.n_listed : tgt.n;
     if ( ch.n_listed )
     {
-        ch.seq = max( 1, min( ch.seq, (int)( n_queries / ( 4 * Q_WARPS * (int64_t)gridDim.x ) ) ) );
-        ch.n_big = n_queries;
+        int64_t const warps = Q_WARPS * (int64_t)gridDim.x;
+        ch.seq = max( 1, (int)min( (int64_t)ch.seq, n_queries / ( 4 * warps ) ) );
+        ch.n_big = n_queries > warps * ch.seq ? ( n_queries - warps * ch.seq ) / ch.seq : 0;
     }
     for ( ;; )
     {
@@ -1922,6 +1923,31 @@ __device__ __forceinline__ float window_bound( TreeView const &tr, uint32_t code
             v |= 1u << bit;
     }
     return v < 0x7f800000u ? __uint_as_float( v ) : __int_as_float( 0x7f800000 );
+}
+
+// Counters of a search, zeroed: the next chunk of k_knn over all queries, of
+// k_knn_lanes and of k_knn over the list; the list's length with the failed and
+// the settled batches behind it; the queries left to k_knn as they are.
+enum : int
+{
+    KNN_CHUNK,
+    KNN_LANES_CHUNK,
+    KNN_LIST_CHUNK,
+    KNN_LISTED,
+    KNN_FAILED,
+    KNN_SETTLED,
+    KNN_ALL,
+    KNN_WORDS
+};
+
+// After the pilot: a cloud that does not suit is k_knn's as a whole, in its own
+// order and chunks (as a list, whose runs of queries lie where the warps came to
+// pass them on, it took 2 to 11% longer); k_knn_lanes then finds no chunk.
+__global__ void k_knn_verdict( unsigned *words, int64_t n )
+{
+    bool const unfit = words[KNN_FAILED] > words[KNN_SETTLED] / 4u;
+    words[KNN_ALL] = unfit ? (unsigned)n : 0u;
+    words[KNN_LANES_CHUNK] = unfit ? (unsigned)( ( n + 31 ) / 32 ) : 0u;
 }
 
 template <int CAP>
@@ -2758,9 +2784,8 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
     int64_t const n_chunks = n_big + ( tgt.n - n_big * seq + tail - 1 ) / tail;
     int64_t const warps = n_chunks < resident ? n_chunks : resident;
     unsigned const blocks = blocks_for( warps, Q_WARPS );
-    // chunk counters of k_knn and of k_knn_lanes; the list's length, failed and settled batches
-    DeviceBuffer<unsigned> next( 5, s );
-    DTK_CUDA_OR_THROW( cudaMemsetAsync( next.get(), 0, 5 * sizeof( unsigned ), s ) );
+    DeviceBuffer<unsigned> next( KNN_WORDS, s );
+    DTK_CUDA_OR_THROW( cudaMemsetAsync( next.get(), 0, KNN_WORDS * sizeof( unsigned ), s ) );
     DeviceBuffer<Query> qrec( tgt.n, s );
     // 32 queries a warp, in columns of 40 for rows up to 16 and of 72 above,
     // from 6 and 24 batches a resident warp on: below that the pilot and the
@@ -2786,24 +2811,31 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
         DeviceBuffer<float> bounds( tgt.n, s );
         auto const kernel = row <= 16 ? k_knn_lanes<KL_CAP_SHORT> : k_knn_lanes<KL_CAP>;
         int64_t const batches = ( tgt.n + 31 ) / 32;
-        kernel<<<KL_PILOT / KL_WARPS, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, 1, next.get() + 1,
+        unsigned *const words = next.get();
+        kernel<<<KL_PILOT / KL_WARPS, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, 1, words + KNN_LANES_CHUNK,
                                                            batches / KL_PILOT, growth, offset, idx, pos, list.get(),
-                                                           bounds.get(), next.get() + 2, status );
+                                                           bounds.get(), words + KNN_LISTED, status );
         check_launch( "k_knn_lanes(pilot)" );
-        kernel<<<lane_blocks, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, per_warp, next.get() + 1, 0,
-                                                   growth, offset, idx, pos, list.get(), bounds.get(), next.get() + 2,
-                                                   status );
+        k_knn_verdict<<<1, 1, 0, s>>>( words, tgt.n );
+        check_launch( "k_knn_verdict" );
+        kernel<<<lane_blocks, KL_THREADS, 0, s>>>( view_of( tree ), tgt, order, row, per_warp, words + KNN_LANES_CHUNK,
+                                                   0, growth, offset, idx, pos, list.get(), bounds.get(),
+                                                   words + KNN_LISTED, status );
         check_launch( "k_knn_lanes" );
-        // what it left
-        k_query_frame<<<8 * num_sms(), 256, 0, s>>>( tgt, list.get(), tree.scene.get(), qrec.get(), next.get() + 2 );
-        check_launch( "k_query_frame" );
-        KnnChunks const rest{Q_SEQ, 0, next.get(), next.get() + 2, bounds.get()};
-        k_knn<false><<<num_sms() * KNN_BLOCKS_PER_SM, Q_WARPS * 32, 0, s>>>(
-            view_of( tree ), tgt, list.get(), qrec.get(), k, rest, gv, offset, idx, pos, status );
-        check_launch( "k_knn" );
+        // all queries, or what it left (one of the two launches is empty)
+        auto const general = [&]( uint32_t const *queries, float const *guesses, unsigned *count, unsigned *chunk ) {
+            k_query_frame<<<8 * num_sms(), 256, 0, s>>>( tgt, queries, tree.scene.get(), qrec.get(), count );
+            check_launch( "k_query_frame" );
+            k_knn<false><<<num_sms() * KNN_BLOCKS_PER_SM, Q_WARPS * 32, 0, s>>>(
+                view_of( tree ), tgt, queries, qrec.get(), k, KnnChunks{Q_SEQ, 0, chunk, count, guesses}, gv, offset,
+                idx, pos, status );
+            check_launch( "k_knn" );
+        };
+        general( order, nullptr, words + KNN_ALL, words + KNN_CHUNK );
+        general( list.get(), bounds.get(), words + KNN_LISTED, words + KNN_LIST_CHUNK );
         return;
     }
-    KnnChunks const ch{seq, n_big, next.get(), nullptr, nullptr};
+    KnnChunks const ch{seq, n_big, next.get() + KNN_CHUNK, nullptr, nullptr};
     k_query_frame<<<blocks_for( tgt.n, 256 ), 256, 0, s>>>( tgt, order, tree.scene.get(), qrec.get() );
     check_launch( "k_query_frame" );
     if ( groups.tgt_grp )
