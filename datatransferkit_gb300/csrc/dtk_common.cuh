@@ -480,6 +480,8 @@ struct Lbvh
     DeviceBuffer<float4> wide_cell;   // per wide node: its Morton cell as a box (lo + parent, hi), inset
     int64_t n_wide = 0;
     int wide_levels = 0;              // the deepest wide node's level (root 0)
+    double shared_nodes = 0.0;        // part of the binary nodes whose leaves lie in one Morton cell
+    int64_t most_shared = 0;          // the most leaves in one
     DeviceBuffer<float4> root_box;    // box of the whole tree (2 float4)
     DeviceBuffer<double> scene;       // lo[3], Morton scale[3], hi[3], centre[3], bound S, FP32 lo/scale
 };

@@ -605,10 +605,13 @@ __device__ __forceinline__ void load_wide( float4 const *wide, int2 const *wide_
     }
 }
 
-// Wide nodes: the binary nodes at depths 0, 3, 6, ...; max_depth gets the
-// largest binary depth (the wide levels bound the traversal stacks).
-__global__ void k_depth_flags( int64_t ni, int const *parent_node, int64_t *flag, unsigned *max_depth,
-                               unsigned *status )
+// Wide nodes: the binary nodes at depths 0, 3, 6, ...; shape gets the largest
+// binary depth (the wide levels bound the traversal stacks), the nodes whose
+// leaves all lie in one Morton cell, split by their order alone (their boxes
+// overlap), and the most leaves of such a node.
+__global__ void k_depth_flags( int64_t ni, int const *parent_node, uint32_t const *codes, uint32_t const *grp,
+                               int32_t const *leaf_start, int const *range_lo, int const *range_hi, int64_t *flag,
+                               unsigned *shape, unsigned *status )
 {
     int64_t const i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if ( i >= ni )
@@ -628,8 +631,19 @@ __global__ void k_depth_flags( int64_t ni, int const *parent_node, int64_t *flag
     flag[i] = d % 3 == 0 ? 1 : 0;
     unsigned const m = __activemask();
     unsigned const dm = __reduce_max_sync( m, (unsigned)d );
+    int const lo = range_lo[i], hi = range_hi[i];
+    bool const one_cell = leaf_key( codes, grp, leaf_start, lo ) == leaf_key( codes, grp, leaf_start, hi );
+    unsigned const shared = __popc( __ballot_sync( m, one_cell ) );
+    unsigned const most = __reduce_max_sync( m, one_cell ? (unsigned)( hi - lo + 1 ) : 0u );
     if ( ( threadIdx.x & 31 ) == __ffs( m ) - 1 )
-        atomicMax( max_depth, dm );
+    {
+        atomicMax( shape, dm );
+        if ( shared )
+        {
+            atomicAdd( shape + 1, shared );
+            atomicMax( shape + 2, most );
+        }
+    }
 }
 
 __device__ __forceinline__ uint32_t compact10( uint32_t v )
@@ -2651,19 +2665,22 @@ void build_lbvh( PointsView src, Lbvh &tree, unsigned *status, cudaStream_t s,
     if ( ni > 0 )
     {
         DeviceBuffer<int64_t> flag( ni, s ), widx( ni + 1, s );
-        DeviceBuffer<unsigned> max_depth( 1, s );
-        DTK_CUDA_OR_THROW( cudaMemsetAsync( max_depth.get(), 0, sizeof( unsigned ), s ) );
-        k_depth_flags<<<blocks_for( ni, 256 ), 256, 0, s>>>( ni, parent_node.get(), flag.get(), max_depth.get(),
-                                                             status );
+        unsigned shape[3] = {0, 0, 0};
+        DeviceBuffer<unsigned> d_shape( 3, s );
+        DTK_CUDA_OR_THROW( cudaMemsetAsync( d_shape.get(), 0, sizeof( shape ), s ) );
+        k_depth_flags<<<blocks_for( ni, 256 ), 256, 0, s>>>( ni, parent_node.get(), tree.codes.get(), tree.grp.get(),
+                                                             tree.leaf_start.get(), range_lo.get(), range_hi.get(),
+                                                             flag.get(), d_shape.get(), status );
         check_launch( "k_depth_flags" );
         exclusive_scan_i64( flag.get(), widx.get(), ni, s );
         int64_t nw = 0;
-        unsigned depth = 0;
         DTK_CUDA_OR_THROW( cudaMemcpyAsync( &nw, widx.get() + ni, sizeof( int64_t ), cudaMemcpyDeviceToHost, s ) );
-        DTK_CUDA_OR_THROW( cudaMemcpyAsync( &depth, max_depth.get(), sizeof( unsigned ), cudaMemcpyDeviceToHost, s ) );
+        DTK_CUDA_OR_THROW( cudaMemcpyAsync( shape, d_shape.get(), sizeof( shape ), cudaMemcpyDeviceToHost, s ) );
         DTK_CUDA_OR_THROW( cudaStreamSynchronize( s ) );
         tree.n_wide = nw;
-        tree.wide_levels = (int)( depth / 3 );
+        tree.wide_levels = (int)( shape[0] / 3 );
+        tree.shared_nodes = (double)shape[1] / (double)ni;
+        tree.most_shared = shape[2];
         tree.wide.allocate( 16 * std::max<int64_t>( 1, nw ), s );
         tree.wide_range.allocate( 8 * std::max<int64_t>( 1, nw ), s );
         k_collapse<<<blocks_for( ni, 128 ), 128, 0, s>>>( ni, tree.nodes.get(), flag.get(), widx.get(),
@@ -2761,9 +2778,16 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
     // run three waves of its resident warps or more: with fewer queries it
     // spreads them over more lanes (2M sources and 20k queries 828 against
     // 859 us with the tree; 30k and 30k 484 against 454, 2M and 2M 3.97
-    // against 1.86 ms).
+    // against 1.86 ms).  Leaves of one Morton cell overlap, and a query next to
+    // them scans them all: 2 ms for 350 of them by a lane alone, however few such
+    // queries there are, so enough queries have to share that time, and not all
+    // of the cloud may be so (ms, k_knn / k_nearest: coordinates to the fourth
+    // power, 2M sources and 350 leaves, 125k queries 1.65 / 2.74, 500k 3.16 /
+    // 2.99, 2M 7.80 / 3.64; 50 clusters, as many queries: 1M sources, 72% shared,
+    // 5.03 / 3.97, 4M, 89%, 1M queries 10.4 / 11.9).
     if ( k == 1 && !groups.tgt_grp && tree.wide_levels <= NN_LEVELS &&
-         tgt.n >= 3 * (int64_t)num_sms() * KNN_BLOCKS_PER_SM * Q_WARPS )
+         tgt.n >= 3 * (int64_t)num_sms() * KNN_BLOCKS_PER_SM * Q_WARPS && tgt.n >= 1500 * tree.most_shared &&
+         tree.shared_nodes <= 0.8 )
     {
         k_nearest<<<blocks_for( tgt.n, NN_THREADS ), NN_THREADS, 0, s>>>( view_of( tree ), tgt, order, idx, pos,
                                                                           status );
