@@ -356,11 +356,13 @@ __device__ __forceinline__ int delta( uint32_t const *codes, uint32_t const *grp
 
 // Internal node i covers leaves [lo[i], hi[i]]; its left child covers
 // [lo, gamma] and its right child [gamma + 1, hi], gamma being the index of
-// the left child (leaf or internal, Karras 2012).
+// the left child (leaf or internal, Karras 2012).  shared gets the nodes whose
+// leaves all lie in one Morton cell, split by their order alone (their boxes
+// overlap), and the most leaves of such a node.
 __global__ void k_karras( uint32_t const *codes, uint32_t const *grp, int32_t const *leaf_start, int64_t nl,
                           int *left,
                           int *right, int *parent_node, int *parent_leaf, int *range_lo,
-                          int *range_hi )
+                          int *range_hi, unsigned *shared )
 {
     int64_t const i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if ( i >= nl - 1 )
@@ -411,6 +413,16 @@ __global__ void k_karras( uint32_t const *codes, uint32_t const *grp, int32_t co
     right[i] = rc;
     range_lo[i] = (int)lo;
     range_hi[i] = (int)hi;
+    unsigned const m = __activemask(), cells = __ballot_sync( m, dnode >= 64 ); // (equal keys)
+    if ( cells )
+    {
+        unsigned const most = __reduce_max_sync( m, dnode >= 64 ? (unsigned)( hi - lo + 1 ) : 0u );
+        if ( ( threadIdx.x & 31 ) == __ffs( m ) - 1 )
+        {
+            atomicAdd( shared, (unsigned)__popc( cells ) );
+            atomicMax( shared + 1, most );
+        }
+    }
 }
 
 struct Box
@@ -605,13 +617,10 @@ __device__ __forceinline__ void load_wide( float4 const *wide, int2 const *wide_
     }
 }
 
-// Wide nodes: the binary nodes at depths 0, 3, 6, ...; shape gets the largest
-// binary depth (the wide levels bound the traversal stacks), the nodes whose
-// leaves all lie in one Morton cell, split by their order alone (their boxes
-// overlap), and the most leaves of such a node.
-__global__ void k_depth_flags( int64_t ni, int const *parent_node, uint32_t const *codes, uint32_t const *grp,
-                               int32_t const *leaf_start, int const *range_lo, int const *range_hi, int64_t *flag,
-                               unsigned *shape, unsigned *status )
+// Wide nodes: the binary nodes at depths 0, 3, 6, ...; max_depth gets the
+// largest binary depth (the wide levels bound the traversal stacks).
+__global__ void k_depth_flags( int64_t ni, int const *parent_node, int64_t *flag, unsigned *max_depth,
+                               unsigned *status )
 {
     int64_t const i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if ( i >= ni )
@@ -631,19 +640,8 @@ __global__ void k_depth_flags( int64_t ni, int const *parent_node, uint32_t cons
     flag[i] = d % 3 == 0 ? 1 : 0;
     unsigned const m = __activemask();
     unsigned const dm = __reduce_max_sync( m, (unsigned)d );
-    int const lo = range_lo[i], hi = range_hi[i];
-    bool const one_cell = leaf_key( codes, grp, leaf_start, lo ) == leaf_key( codes, grp, leaf_start, hi );
-    unsigned const shared = __popc( __ballot_sync( m, one_cell ) );
-    unsigned const most = __reduce_max_sync( m, one_cell ? (unsigned)( hi - lo + 1 ) : 0u );
     if ( ( threadIdx.x & 31 ) == __ffs( m ) - 1 )
-    {
-        atomicMax( shape, dm );
-        if ( shared )
-        {
-            atomicAdd( shape + 1, shared );
-            atomicMax( shape + 2, most );
-        }
-    }
+        atomicMax( max_depth, dm );
 }
 
 __device__ __forceinline__ uint32_t compact10( uint32_t v )
@@ -2644,14 +2642,16 @@ void build_lbvh( PointsView src, Lbvh &tree, unsigned *status, cudaStream_t s,
     DeviceBuffer<int> left( std::max<int64_t>( 1, ni ), s ), right( std::max<int64_t>( 1, ni ), s ),
         parent_node( std::max<int64_t>( 1, ni ), s ), parent_leaf( nl, s ),
         range_lo( std::max<int64_t>( 1, ni ), s ), range_hi( std::max<int64_t>( 1, ni ), s );
-    DeviceBuffer<unsigned> flags( std::max<int64_t>( 1, ni ), s );
+    // the nodes' visits, then the tree's shape: shared nodes, the most leaves of one, the largest depth
+    DeviceBuffer<unsigned> flags( ni + 3, s );
     DTK_CUDA_OR_THROW( cudaMemsetAsync( flags.get(), 0, flags.n * sizeof( unsigned ), s ) );
+    unsigned *const d_shape = flags.get() + ni;
     if ( ni > 0 )
     {
         k_karras<<<blocks_for( ni, 256 ), 256, 0, s>>>( tree.codes.get(), tree.grp.get(), tree.leaf_start.get(),
                                                           nl, left.get(),
                                                           right.get(), parent_node.get(), parent_leaf.get(),
-                                                          range_lo.get(), range_hi.get() );
+                                                          range_lo.get(), range_hi.get(), d_shape );
         check_launch( "k_karras" );
         k_pack_children<<<blocks_for( ni, 256 ), 256, 0, s>>>( ni, left.get(), right.get(), range_lo.get(),
                                                                  range_hi.get(), tree.nodes.get() );
@@ -2665,22 +2665,18 @@ void build_lbvh( PointsView src, Lbvh &tree, unsigned *status, cudaStream_t s,
     if ( ni > 0 )
     {
         DeviceBuffer<int64_t> flag( ni, s ), widx( ni + 1, s );
-        unsigned shape[3] = {0, 0, 0};
-        DeviceBuffer<unsigned> d_shape( 3, s );
-        DTK_CUDA_OR_THROW( cudaMemsetAsync( d_shape.get(), 0, sizeof( shape ), s ) );
-        k_depth_flags<<<blocks_for( ni, 256 ), 256, 0, s>>>( ni, parent_node.get(), tree.codes.get(), tree.grp.get(),
-                                                             tree.leaf_start.get(), range_lo.get(), range_hi.get(),
-                                                             flag.get(), d_shape.get(), status );
+        k_depth_flags<<<blocks_for( ni, 256 ), 256, 0, s>>>( ni, parent_node.get(), flag.get(), d_shape + 2, status );
         check_launch( "k_depth_flags" );
         exclusive_scan_i64( flag.get(), widx.get(), ni, s );
         int64_t nw = 0;
+        unsigned shape[3] = {0, 0, 0};
         DTK_CUDA_OR_THROW( cudaMemcpyAsync( &nw, widx.get() + ni, sizeof( int64_t ), cudaMemcpyDeviceToHost, s ) );
-        DTK_CUDA_OR_THROW( cudaMemcpyAsync( shape, d_shape.get(), sizeof( shape ), cudaMemcpyDeviceToHost, s ) );
+        DTK_CUDA_OR_THROW( cudaMemcpyAsync( shape, d_shape, sizeof( shape ), cudaMemcpyDeviceToHost, s ) );
         DTK_CUDA_OR_THROW( cudaStreamSynchronize( s ) );
         tree.n_wide = nw;
-        tree.wide_levels = (int)( shape[0] / 3 );
-        tree.shared_nodes = (double)shape[1] / (double)ni;
-        tree.most_shared = shape[2];
+        tree.wide_levels = (int)( shape[2] / 3 );
+        tree.shared_nodes = (double)shape[0] / (double)ni;
+        tree.most_shared = shape[1];
         tree.wide.allocate( 16 * std::max<int64_t>( 1, nw ), s );
         tree.wide_range.allocate( 8 * std::max<int64_t>( 1, nw ), s );
         k_collapse<<<blocks_for( ni, 128 ), 128, 0, s>>>( ni, tree.nodes.get(), flag.get(), widx.get(),
