@@ -525,11 +525,18 @@ __host__ __device__ __forceinline__ void fx_pivots( State const &st, float ( &a 
 // FP32 is (each bounds it from above, as the smallest eigenvalue of a leading
 // block does).  Without it clouds of so small a scale paid for both forms: 300k
 // quadratic targets in a cube of edge 0.01 took 9.8 ms, now 8.6 (FP64 alone
-// 7.4); at edge 1, where no matrix is handed back, it costs 0.04 of 8.25 ms.
+// 7.4).
 template <int M, class State>
 __host__ __device__ __forceinline__ bool fx_truncates( State const &st )
 {
     using Lay = FxLayout<M>;
+    // (a pivot is 2^-17 2^(2 d) at least: most clouds end here)
+    bool small = false;
+#pragma unroll
+    for ( int k = 0; k < M; ++k )
+        small |= 2 * st.exp( k ) - 17 < FX_TRUNCATE;
+    if ( !small )
+        return false;
     float a[M][M]; // the upper triangle, in units of 2^(d_i + d_j)
     bool truncates = false;
 #pragma unroll
