@@ -93,8 +93,9 @@ bool is_pow2( int v ) { return v > 0 && ( v & ( v - 1 ) ) == 0; }
 // row's neighbours sit in a few sectors of an L2-resident array instead of 32
 // scattered ones; c_j (hi_j + lo_j) is summed in double-float arithmetic on the
 // FP32 pipe (TwoProd / TwoSum, the compensated scheme of the mixed setup): the
-// FP32 coefficients are the only rounding left, as with an FP64 sum, for values
-// in FP32's range.
+// FP32 coefficients are the only rounding left, as with an FP64 sum.  A row whose
+// sum says that FP32's range was not enough (not finite, or below 2^-60, where a
+// term's low part nears the subnormals) is summed again in FP64 from the field.
 //
 // FP64 sums, for the FP64 form and for fields of several components in both (a
 // double-float has FP32's range and 48 bits): FP64 FMAs, whose pipe bounds them
@@ -114,6 +115,12 @@ bool is_pow2( int v ) { return v > 0 && ( v & ( v - 1 ) ) == 0; }
 namespace
 {
 
+// the biased exponent (integer pipe)
+__device__ __forceinline__ int exponent_of( double v )
+{
+    return ( __double2hiint( v ) >> 20 ) & 0x7ff;
+}
+
 __device__ __forceinline__ void two_sum( float a, float b, float &s, float &e )
 {
     s = __fadd_rn( a, b );
@@ -128,7 +135,8 @@ __device__ __forceinline__ void two_prod( float a, float b, float &p, float &e )
 }
 
 // sorted[p] = values[perm[p]] (perm null: the identity) as a double (FP64
-// form) or a double-float
+// form) or a double-float; NaN for a value that FP32 products could lose (its
+// rows are summed in FP64)
 __global__ void k_permute_values( int64_t n, uint32_t const *__restrict__ perm, double const *__restrict__ values,
                                   double *__restrict__ sorted64, float2 *__restrict__ sorted32 )
 {
@@ -138,8 +146,12 @@ __global__ void k_permute_values( int64_t n, uint32_t const *__restrict__ perm, 
     double const v = __ldg( values + ( perm ? (int64_t)__ldg( perm + p ) : p ) );
     if ( sorted32 )
     {
-        float const hi = __double2float_rn( v );
-        sorted32[p] = make_float2( hi, __double2float_rn( v - (double)hi ) );
+        float hi = __double2float_rn( v );
+        float const lo = __double2float_rn( v - (double)hi );
+        // 0 < |v| < 2^-100
+        if ( exponent_of( v ) < 1023 - 100 && ( __double_as_longlong( v ) << 1 ) != 0 )
+            hi = __int_as_float( 0x7fffffff );
+        sorted32[p] = make_float2( hi, lo );
     }
     else
         sorted64[p] = v;
@@ -156,9 +168,9 @@ __device__ __forceinline__ void df_axpy( float c, float2 v, float &s, float &cs 
     cs = __fadd_rn( cs, __fadd_rn( f, e ) );
 }
 
-// The double-floats (s, cs) of a group of L lanes added up.
+// The double-floats (s, cs) of a group of L lanes added up, in every lane.
 template <int L>
-__device__ __forceinline__ double df_group_sum( float s, float cs )
+__device__ __forceinline__ void df_group_sum( float &s, float &cs )
 {
 #pragma unroll
     for ( int o = L / 2; o > 0; o >>= 1 )
@@ -169,7 +181,6 @@ __device__ __forceinline__ double df_group_sum( float s, float cs )
         s = t;
         cs = __fadd_rn( cs, __fadd_rn( oc, f ) );
     }
-    return (double)s + (double)cs;
 }
 
 // Exactly (double)c on the integer pipe: a conversion takes the FP64 pipe 64
@@ -208,12 +219,25 @@ __device__ __forceinline__ void load_coeff4( float const *p, double *c )
     c[3] = widen( v.w );
 }
 
+// A row's sum in FP64 from the field (apart, so that the callers' loads stay
+// together).
+__device__ __noinline__ double row_sum64( int n, int32_t const *pos, float const *coeff, double const *values,
+                                          uint32_t const *perm )
+{
+    double sum = 0.0;
+    for ( int j = 0; j < n; ++j )
+        sum = fma( (double)coeff[j], values[perm ? (int64_t)perm[pos[j]] : pos[j]], sum );
+    return sum;
+}
+
 // Mixed form, one component: L lanes per row, each lane EPL consecutive entries
-// (EPL a multiple of 4).
+// (EPL a multiple of 4).  values, perm: the field and its order, for the rows
+// that FP32's range does not hold.
 template <int L, int EPL>
 __global__ void __launch_bounds__( 256 )
     k_apply_pos( int64_t n_tgt, int32_t const *__restrict__ pos, float const *__restrict__ coeff,
-                 float2 const *__restrict__ sorted, double *__restrict__ target, uint32_t const *__restrict__ order )
+                 float2 const *__restrict__ sorted, double const *__restrict__ values,
+                 uint32_t const *__restrict__ perm, double *__restrict__ target, uint32_t const *__restrict__ order )
 {
     constexpr int R = EPL * L;
     int64_t const gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -235,9 +259,13 @@ __global__ void __launch_bounds__( 256 )
             df_axpy( c.w, __ldg( sorted + ix.w ), s, cs );
         }
     }
-    double const sum = df_group_sum<L>( s, cs );
+    df_group_sum<L>( s, cs );
     if ( row < n_tgt && sub == 0 )
-        target[row] = sum;
+    {
+        float const size = fabsf( s );
+        bool const held = ( size >= 8.6736174e-19f && size <= 3.4028235e38f ) || ( s == 0.f && cs == 0.f ); // 2^-60
+        target[row] = held ? (double)s + (double)cs : row_sum64( R, pos + row * R, coeff + row * R, values, perm );
+    }
 }
 
 // FP64 sums of CB components from c0 on: L lanes take ROWS rows, each lane EPL
@@ -351,16 +379,17 @@ __global__ void k_permute_fields( FieldView in, int64_t c0, int nc, uint32_t con
             sorted[nc * p + k] = __ldg( v + k * in.cs );
 }
 
-// fn( lanes a row, entries a lane ) of row length R, with SHORTEST entries a
-// lane for rows of 8
-template <int SHORTEST, class Fn>
+// fn( lanes a row, entries a lane ) of row length R (a lane of 8 entries reads a
+// sector in two loads, which has to stay in L1 between them: rows of 8 by two
+// lanes)
+template <class Fn>
 void for_row_shape( int R, Fn const &fn )
 {
     std::integral_constant<int, 8> const eight;
     switch ( R )
     {
     case 4: fn( std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{} ); break;
-    case 8: fn( std::integral_constant<int, 8 / SHORTEST>{}, std::integral_constant<int, SHORTEST>{} ); break;
+    case 8: fn( std::integral_constant<int, 2>{}, std::integral_constant<int, 4>{} ); break;
     case 16: fn( std::integral_constant<int, 2>{}, eight ); break;
     case 32: fn( std::integral_constant<int, 4>{}, eight ); break;
     case 64: fn( std::integral_constant<int, 8>{}, eight ); break;
@@ -381,7 +410,7 @@ void launch_rows64( int64_t n_rows, int R, int32_t const *at, Coeff const *coeff
     int64_t const n_full = in.n_comp - groups * ( CB - 1 );
     bool const packed = in.n_comp == CB && in.ps == CB && ( CB == 1 || in.cs == 1 );
     bool const several = n_rows >= 100000 && ( CB >= 3 || ( CB == 2 && sorted ) );
-    for_row_shape<4>( R, [&]( auto l, auto epl ) {
+    for_row_shape( R, [&]( auto l, auto epl ) {
         constexpr int L = decltype( l )::value, EPL = decltype( epl )::value;
         constexpr int MOST = CB == 1 || L == 1 ? 1 : L < 4 ? L : 4;
         auto const run = [&]( auto rows, auto is_packed ) {
@@ -455,7 +484,7 @@ SortedValues permute_values( int64_t n_src, uint32_t const *perm, double const *
 }
 
 void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double const *coeff64, float const *coeff32,
-                SortedValues const &v, double *target, cudaStream_t s, uint32_t const *order )
+                SortedValues const &v, double const *values, uint32_t const *perm, double *target, cudaStream_t s, uint32_t const *order )
 {
     if ( n_rows == 0 )
         return;
@@ -465,10 +494,11 @@ void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double cons
                       rank1( nullptr, target, n_rows ), true, s, order );
         return;
     }
-    for_row_shape<8>( uniform_row, [&]( auto l, auto epl ) {
+    for_row_shape( uniform_row, [&]( auto l, auto epl ) {
         constexpr int L = decltype( l )::value, EPL = decltype( epl )::value;
         k_apply_pos<L, EPL><<<(unsigned)( ( n_rows * L + 255 ) / 256 ), 256, 0, s>>>( n_rows, pos, coeff32,
-                                                                                      v.v32.get(), target, order );
+                                                                                      v.v32.get(), values, perm,
+                                                                                      target, order );
         check_launch( "k_apply_pos" );
     } );
 }
@@ -485,8 +515,9 @@ void apply_sorted( int64_t n_tgt, int uniform_row, int32_t const *idx, int32_t c
                       rank1( nullptr, target, n_tgt ), false, s, order );
         return;
     }
-    SortedValues const v = permute_values( n_src, pos ? perm : nullptr, values, true, s );
-    apply_pos( n_tgt, uniform_row, pos ? pos : idx, nullptr, coeff32, v, target, s, order );
+    uint32_t const *const by = pos ? perm : nullptr;
+    SortedValues const v = permute_values( n_src, by, values, true, s );
+    apply_pos( n_tgt, uniform_row, pos ? pos : idx, nullptr, coeff32, v, values, by, target, s, order );
 }
 
 void apply_sorted_multi( int64_t n_tgt, int uniform_row, int32_t const *idx, int32_t const *pos,

@@ -665,7 +665,8 @@ dtk_status dtk_mls_transfer_host( const dtk_mls_options *opts, const double *src
             int64_t const r1 = std::min( n_tgt, r0 + per );
             if ( by_pos )
                 apply_pos( r1 - r0, R, h->pos.get() + r0 * R, h->coeff64.get() ? h->coeff64.get() + r0 * R : nullptr,
-                           h->coeff32.get() ? h->coeff32.get() + r0 * R : nullptr, sorted, d_out.get() + r0, s );
+                           h->coeff32.get() ? h->coeff32.get() + r0 * R : nullptr, sorted, d_vals.get(),
+                           h->perm.get(), d_out.get() + r0, s );
             else if ( R > 0 ) // uniform rows: offset[i] = i R also indexes the shifted slice
                 apply_csr( r1 - r0, h->offset.get(), h->idx.get() + r0 * R,
                            h->coeff64.get() ? h->coeff64.get() + r0 * R : nullptr,

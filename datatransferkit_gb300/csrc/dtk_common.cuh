@@ -717,9 +717,11 @@ SortedValues permute_values( int64_t n_src, uint32_t const *perm, double const *
                              cudaStream_t s );
 // n_rows uniform rows starting at pos / coeff (a slice of the operator's),
 // taken in the given order (the targets' Morton order: consecutive rows then
-// share most of their neighbours' values in L1) or in row order
+// share most of their neighbours' values in L1) or in row order; values, perm:
+// what v was made from
 void apply_pos( int64_t n_rows, int uniform_row, int32_t const *pos, double const *coeff64, float const *coeff32,
-                SortedValues const &v, double *target, cudaStream_t s, uint32_t const *order = nullptr );
+                SortedValues const &v, double const *values, uint32_t const *perm, double *target, cudaStream_t s,
+                uint32_t const *order = nullptr );
 // A whole operator with uniform rows, by index (idx) or, where pos is not null
 // and it pays, by sorted position on a copy of the values; the FP64 sums are the
 // same bits either way.  A mixed operator's rank-1 field is summed in
