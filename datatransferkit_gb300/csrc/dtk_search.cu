@@ -2807,19 +2807,24 @@ void knn_query( Lbvh const &tree, PointsView tgt, uint32_t const *order, int k,
     DeviceBuffer<unsigned> next( KNN_WORDS, s );
     DTK_CUDA_OR_THROW( cudaMemsetAsync( next.get(), 0, KNN_WORDS * sizeof( unsigned ), s ) );
     DeviceBuffer<Query> qrec( tgt.n, s );
-    // 32 queries a warp, in columns of 40 for rows up to 16 and of 72 above,
-    // from 6 and 24 batches a resident warp on: below that the pilot and the
-    // warps' first batches, whose bounds are rough, take what the others save.
-    // Search with the tree, k_knn alone against this: k = 8, 800k targets 1.97
-    // / 1.73 ms, 2M 4.28 / 3.10, 8M 15.2 / 9.6; k = 20, 2M 4.39 / 4.00 (1M 2.46
-    // / 2.31), 8M 15.6 / 13.1; k = 32, 1M 2.77 / 2.93, 2M 5.01 / 4.89, 8M 17.5
-    // / 15.8.  At 3M and k = 20: grid 7.5 / 6.9, sphere 5.5 / 5.1, clusters 6.8
-    // / 7.2, duplicates 10.1 / 9.6, targets far outside 5.6 / 5.7, coordinates
-    // to the fourth power 14.2 / 15.4.
+    // 32 queries a warp, in columns of 40 for rows up to 16 and of 72 above.
+    // Below some hundred batches a resident warp the pilot and the warps' first
+    // batches, whose bounds are rough, take what the others save; the longer the
+    // rows the later it pays, and on graded clouds later than on uniform ones.
+    // Time of the queries over k_knn's, uniform / 144^3 grid / squared
+    // coordinates / Gaussian / sphere / sevenfold duplicates:
+    //   k = 12, 1M targets  0.88 0.86 1.02 1.18 0.86 1.18
+    //   k = 16, 1M          0.95 0.82 1.10 1.21 0.92 1.31,  2M 0.79 0.73 0.88 0.99 0.76 1.24
+    //   k = 20, 2M          0.87 0.83 1.00 1.08 0.94 0.96
+    //   k = 28, 2M          0.91 0.84 1.07 1.12 1.05 0.99,  8M 0.85 0.77 1.01 1.00 0.91 0.91
+    //   k = 32, 2M          0.97 0.87 1.13 1.17 1.13 1.25,  4M 0.93 0.84 1.11 1.06 1.08 1.22,
+    //           8M          0.88 0.76 1.07 1.03 0.98 1.17
+    // The lines lie where the mean of these is about 1.
     int const row = (int)std::min<int64_t>( k, tree.n );
     int const lane_blocks = num_sms() * ( row <= 16 ? KL_BLOCKS_SHORT : KL_BLOCKS );
     int64_t const lane_warps = (int64_t)lane_blocks * KL_WARPS;
-    if ( !groups.tgt_grp && tree.wide_levels <= NN_LEVELS && tgt.n >= ( row <= 16 ? 192 : 768 ) * lane_warps )
+    int const per_lane_warp = row <= 12 ? 192 : row <= 16 ? 352 : row <= 28 ? 768 : 1600; // queries
+    if ( !groups.tgt_grp && tree.wide_levels <= NN_LEVELS && tgt.n >= per_lane_warp * lane_warps )
     {
         int const cap = row <= 16 ? KL_CAP_SHORT : KL_CAP;
         // the bound from the mean k-th distance: so that it holds 1.6 to 2
