@@ -4,8 +4,8 @@
 //
 // GB300 issues one FP64 warp instruction per 64 cycles per SM sub-partition,
 // a 32 x 32 -> 64 bit integer multiply-add in 4 to 5, and other integer
-// instructions in 2, so 89-bit fixed point is several times faster than FP64,
-// and more precise.  The matrix is kept as
+// instructions in 2, so 89-bit fixed point is several times faster than FP64.
+// The matrix is kept as
 //     E(i, j) = F(i, j) 2^(d_i + d_j),  |F(i, j)| < 1,
 // F in three digits (a signed leading one of 31 bits, two of 29; the diagonal
 // and column 0 of V in two), with a power of two 2^d_i >= sqrt(E(i, i)) per row
@@ -13,20 +13,23 @@
 // the constant and the quadratic terms, and every row keeps its own 89 bits.
 // A rotation multiplies the two rows by four factors of two digits (58 bits
 // after the point, below 4) that carry the change of scale; the product of the
-// lowest digits is left out.  An FP64 rotation rounds at 2^-53 of its
-// operands; this one at 2^-58 of them and at a unit, 2^-89 2^(d_i + d_j), of
-// the result.  (Two digits throughout were a fifth faster, but their unit can
-// be within 2^-12 of the absolute stop for the entries of the constant term: a
-// few of them on the wrong side make one rotation more or less, which moved 1
-// in 1000 targets by up to 1e-8, and running the doubtful ones again, up to 13
-// in 100, took the gain back.)
+// lowest digits is left out.  An FP64 rotation rounds at 2^-53 of its operands;
+// this one at 2^-58 of them and at a unit, 2^-89 2^(d_i + d_j), of the result.
+// Cosine and sine come from the same angle to 2^-58 whatever the pivot block is
+// (the doubles kept of them have c^2 + s^2 = 1 to 3.2e-16 over 7.6M blocks, nearly
+// equal diagonal entries and pivots down to the last unit among them).
+// (Two digits throughout were a fifth faster, but their unit can be within 2^-12
+// of the absolute stop for the entries of the constant term: a few of them on the
+// wrong side make one rotation more or less, which moved 1 in 1000 targets by up
+// to 1e-8, and running the doubtful ones again, up to 13 in 100, took the gain
+// back.)
 //
 // A matrix whose form does not hold is handed back to the FP64 loop, whose
 // truncation decisions rest on its own rounding: a diagonal entry that is not
-// positive, scales out of range, a pivot block singular to 2^-22, a diagonal
-// entry at the absolute truncation threshold at the end, or more rotations
-// than the log takes.  Host builds of the same code are tested against the
-// oracle.
+// positive, scales out of range, a pivot block singular to 2^-22, an eigenvalue
+// at the absolute truncation threshold (found before the first rotation for most
+// such matrices, at the end for the others), or more rotations than the log
+// takes.  Host builds of the same code are tested against the oracle.
 #ifndef DTK_FIXED_CUH
 #define DTK_FIXED_CUH
 
@@ -494,7 +497,7 @@ __host__ __device__ __forceinline__ bool fx_load( State const &st, bool live )
     return st.both( ok );
 }
 
-constexpr int FX_TRUNCATE = -51; // twice DBL_EPSILON's exponent less one
+constexpr int FX_TRUNCATE = -51; // 2^-51, twice DBL_EPSILON
 
 // Pivots K .. of the LDL^T of a, in units of 2^(d_i + d_j).
 template <int M, int K, class State>

@@ -12,12 +12,13 @@
 // latency: about 2.4k warp instructions a rotation at 53% of the issue slots
 // with 10 warps an SM (shared memory), FP64 pipe 27%, ALU 37%.  The loop's code
 // is kept small: with its two halves unrolled the 2M setup takes 44 ms in place
-// of 37.6 (instruction fetch).  2M quadratic targets, k = 32: 84 -> 37.6 ms; 10k, k = 20: 1.20 -> 0.60 ms; 200k rows of 120
-// within a radius: 18.6 -> 8.9 ms; the batched setup of 1.5M targets 26 -> 15.
+// of 37.6 (instruction fetch).  2M quadratic targets, k = 32: 84 -> 37.6 ms; 10k,
+// k = 20: 1.20 -> 0.60 ms; 200k rows of 120 within a radius: 18.6 -> 8.9 ms; the
+// batched setup of 1.5M targets 26 -> 15.
 //
 // Targets the fixed-point form hands back (near-singular moments, scales out
-// of range, a stop within its rounding) are listed, and the FP64 kernel runs
-// them afterwards.
+// of range, eigenvalues at the truncation threshold) are listed, and the FP64
+// kernel runs them afterwards.
 #include "dtk_common.cuh"
 #include "dtk_fixed.cuh"
 #include "dtk_moments.cuh"
@@ -94,7 +95,7 @@ __device__ __forceinline__ double dot_basis( double const *row0, double x, doubl
 
 // The state of a warp's matrices in shared memory, interleaved by matrix: the
 // two leading digits of a number as one 64-bit word, the third digits in a
-// plane of their own, the exponents as bytes (710 B a matrix at M = 10).  With
+// plane of their own, the exponents as bytes (712 B a matrix at M = 10).  With
 // COLS = 32 every lane has a matrix (the fewest instructions: 10 warps an SM).
 // With COLS = 16 lanes c and c + 16 share matrix c, each scanning half of the
 // entries and rotating half of the columns, both computing the angle: 1.4
