@@ -136,7 +136,10 @@ dtk_status dtk_mls_create_from_neighbors(const dtk_mls_options *opts, const doub
  * with its preconditions n_source_values == n_src and n_target_values ==
  * n_tgt (DTK_REQUIRE at :129-130).  Writes every target value; enqueued on
  * `stream`, asynchronous (the reference's apply fences: follow with
- * dtk_stream_synchronize for that behaviour, as the C++ drop-in does). */
+ * dtk_stream_synchronize for that behaviour, as the C++ drop-in does).
+ * The FP64 form sums in FP64; the mixed form in double-float (2^-48 a term)
+ * for rows of 4, 8, 16, 32, 64 or 128 entries, with FP64's range, and in FP64
+ * for the others. */
 dtk_status dtk_mls_apply(dtk_mls_handle h, const double *source_values,
                          int64_t n_source_values, double *target_values,
                          int64_t n_target_values, dtk_stream_t stream);
@@ -288,7 +291,8 @@ dtk_status dtk_mls_import(const void *host_buffer, int64_t bytes,
 /* ---- rank-2 (multi-component) fields ----
  * apply for n x n_comp fields with (point, component) strides in elements:
  * LayoutRight (component fastest): (n_comp, 1); LayoutLeft: (1, n).  Each
- * component is the rank-1 apply of that column.  Extension: the reference's
+ * component is the rank-1 apply of that column, summed in FP64 in both
+ * forms.  Extension: the reference's
  * MLS apply takes rank-1 views (DTK_MovingLeastSquaresOperator_decl.hpp:52-54);
  * its fetch handles rank 2 (DTK_DetailsNearestNeighborOperatorImpl.hpp:53-56,89-93). */
 dtk_status dtk_mls_apply_multi(dtk_mls_handle h, const double *source_values,
