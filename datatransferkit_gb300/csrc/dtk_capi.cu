@@ -632,6 +632,16 @@ dtk_status dtk_mls_transfer_host( const dtk_mls_options *opts, const double *src
         DTK_CUDA_OR_THROW( cudaStreamCreateWithFlags( &side.s2, cudaStreamNonBlocking ) );
         DeviceBuffer<double> d_src( 3 * n_src, s ), d_tgt( std::max<int64_t>( 1, 3 * n_tgt ), s ),
             d_vals( n_src, s ), d_out( std::max<int64_t>( 1, n_tgt ), s );
+        // (where the call throws, the copies on the side stream end before their
+        // buffers are freed on s and the host's are the caller's again)
+        struct Join
+        {
+            cudaStream_t s2;
+            ~Join()
+            {
+                cudaStreamSynchronize( s2 );
+            }
+        } const join{side.s2};
         cudaEvent_t const src_in = side.event(), tgt_ready = side.event(), vals_ready = side.event();
         DTK_CUDA_OR_THROW( cudaMemcpyAsync( d_src.get(), src_host, 3 * n_src * sizeof( double ),
                                             cudaMemcpyHostToDevice, s ) );

@@ -2728,8 +2728,12 @@ void build_tree_and_order( PointsView src, PointsView tgt, Lbvh &tree, DeviceBuf
     {
         cudaStream_t s2 = nullptr;
         cudaEvent_t scene = nullptr, done = nullptr;
+        bool joined = false;
         ~Side()
         {
+            // (a throw on the way: the buffers of both streams are freed next)
+            if ( s2 && !joined )
+                cudaStreamSynchronize( s2 );
             if ( scene )
                 cudaEventDestroy( scene );
             if ( done )
@@ -2751,6 +2755,7 @@ void build_tree_and_order( PointsView src, PointsView tgt, Lbvh &tree, DeviceBuf
         DTK_CUDA_OR_THROW( cudaEventRecord( side.done, side.s2 ) );
     } );
     DTK_CUDA_OR_THROW( cudaStreamWaitEvent( s, side.done, 0 ) );
+    side.joined = true;
     // Points with a NaN or infinite coordinate were flagged by the passes
     // that read them (scene bounds, target Morton codes), whose results stay
     // in range either way; no search runs on them.

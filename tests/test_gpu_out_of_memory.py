@@ -60,3 +60,51 @@ def test_adjoint_after_a_refused_allocation(coords, restore):
 
 def test_failing_allocation_range():
     assert _capi.lib().dtk_set_failing_allocation(-1) == 1
+
+
+@pytest.mark.parametrize("what", ["fp64", "mixed", "radius", "batch", "nearest", "host"])
+def test_calls_after_a_refused_allocation(what, restore):
+    """Every allocation of a call refused in turn: DTK_ERR_OOM, and the same call
+    made right after it gives an undisturbed one's bits."""
+    L = _capi.lib()
+    src = torch.from_numpy(syn.uniform_points(30000, 73)).cuda()
+    tgt = torch.from_numpy(syn.uniform_points(20000, 74)).cuda()
+    vals = torch.from_numpy(syn.smooth_field(src.cpu().numpy())).cuda()
+    basis, rbf = dtk.MultivariatePolynomialBasis(dtk.Linear, 3), dtk.Wendland(2)
+    pinned = [t.cpu().pin_memory() for t in (src, tgt, vals)]
+
+    def call():
+        out = torch.full((len(tgt),), np.nan, dtype=torch.float64, device="cuda")
+        if what == "host":
+            host = out.cpu().pin_memory()
+            dtk.MovingLeastSquaresOperator.transfer_host(None, *pinned, host, rbf, basis, k=8)
+            return host
+        if what == "batch":
+            op = dtk.MovingLeastSquaresBatch([dict(source_points=src, target_points=tgt, rbf=rbf, basis=basis, k=8)])
+        elif what == "nearest":
+            op = dtk.NearestNeighborOperator(None, src, tgt)
+        else:
+            rows = dict(radius=0.06) if what == "radius" else dict(k=8)
+            op = dtk.MovingLeastSquaresOperator(None, src, tgt, rbf, basis,
+                                                precision="mixed" if what == "mixed" else "fp64", **rows)
+        op.apply(vals, out)
+        return out
+
+    want = call()
+    refused = 0
+    for nth in range(1, 400):
+        assert L.dtk_set_failing_allocation(nth) == 0
+        try:
+            got = call()
+        except dtk.DTKError as e:
+            assert e.status == OOM
+            refused += 1
+            got = call()
+        else:
+            assert L.dtk_set_failing_allocation(0) == 0
+            assert torch.equal(got, want)
+            break
+        assert torch.equal(got, want)
+    else:
+        raise AssertionError("the call never ran out of allocations to refuse")
+    assert refused >= 20
